@@ -640,14 +640,178 @@ __global__ void k_brenner(const BrennerParams* P, const BrennerTables* T, BondLi
 
 constexpr int kCijLocal = 128;  // per-thread connectivity table capacity
 
+// Connectivity tables, kCijGroup lanes per atom: cij_build_atom's entries by
+// another route.  The lanes walk the atom's 2-bond paths and their third bonds
+// and lay every path down as a candidate (target, w, code); a candidate stays
+// when no other path to its target has a larger w, or the same w and a smaller
+// code (length, then the slots s1, s2, s3: the reference's order), and the
+// number of smaller targets among those that stay is its place in the row.
+// An atom whose paths or bonds do not fit takes the one-thread build.
+//
+// The candidates lie in a global scratch row per resident group, which stays
+// in L1, and not in shared memory: a kernel that asks for more shared memory
+// than the others makes the SMs change their L1 split between the step's
+// streams, which cost more than the kernel takes (the ethane liquid of 43,680
+// atoms: 313 us a step before, 407 with the rows in shared memory, 306 so).
+// Bound by the instructions of the comparisons on a crystal (52 candidates of
+// a diamond atom), by the latency of the walk's loads on molecules (7).  One
+// thread an atom, its table in local memory: 4.30 ms on 512,000 diamond atoms
+// and 66 us on 64 slabs of 257 atoms; so 0.93 ms and 22 us.
+constexpr int kCijGroup = 8;
+constexpr int kCijThreads = 64;
+constexpr int kCijAtoms = kCijThreads / kCijGroup;
+constexpr int kCijCand = 128;                // candidates per atom (a multiple of 4)
+constexpr int kCijScratch = 4 * kCijCand;    // ints of a group's scratch row: targets, codes, w
+constexpr int kCijNone = 0x7fffffff;         // no target
+
 // Also zeroes the special-pair counters that the special-pair finder after it
 // hands ranges out of.
-__global__ void k_cij(BondList B, CijTable T, unsigned long long* spc_ctr, unsigned int* status)
+__global__ void __launch_bounds__(kCijThreads) k_cij(BondList B, CijTable T, int* scratch,
+                                                     unsigned long long* spc_ctr, unsigned int* status)
 {
   pdl_enter();
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a == 0 && spc_ctr) spc_ctr[0] = spc_ctr[kCtrStride] = spc_ctr[2 * kCtrStride] = 0ull;
-  if (a < B.n) cij_build_atom<kCijLocal>(B, T, a, status);
+  const int tid = threadIdx.x, gl = tid % kCijGroup, lane = tid & 31, gbase = lane - gl;
+  const unsigned gmask = ((1u << kCijGroup) - 1u) << gbase;
+  int* ctgt = scratch + (long)(blockIdx.x * kCijAtoms + tid / kCijGroup) * kCijScratch;
+  unsigned* ccode = reinterpret_cast<unsigned*>(ctgt + kCijCand);
+  double* cw = reinterpret_cast<double*>(ctgt + 2 * kCijCand);
+  if (blockIdx.x == 0 && tid == 0 && spc_ctr) spc_ctr[0] = spc_ctr[kCtrStride] = spc_ctr[2 * kCtrStride] = 0ull;
+  // whole warps stay in the loop: the atoms of a warp's groups are consecutive
+  for (int a0 = blockIdx.x * kCijAtoms + tid / 32 * (32 / kCijGroup); a0 < B.n; a0 += gridDim.x * kCijAtoms) {
+    const int a = a0 + lane / kCijGroup;
+    const bool live = a < B.n;
+    const int nb1 = live ? B.nb[a] : 0;
+    const int q1 = a * B.mb;
+    bool wide = nb1 > kCijGroup || B.mb > 32;
+    // lane s holds the s-th partner, its bond count and weight
+    const bool has = gl < nb1 && !wide;
+    const int k1 = has ? B.bj[q1 + gl] : 0;
+    const double f1 = has ? B.bu[q1 + gl].w : 0.0;
+    const int n1 = has ? B.nb[k1] : 0;
+    int n2 = n1;
+    for (int o = kCijGroup / 2; o > 0; o >>= 1) n2 += __shfl_xor_sync(0xffffffffu, n2, o);
+    const int rounds = (__reduce_max_sync(0xffffffffu, n2) + kCijGroup - 1) / kCijGroup;
+    int n = 0;  // candidates so far (the same on every lane of the group)
+    // appends each lane's candidate, if it has one
+    auto put = [&](bool on, int t, double w, unsigned code) {
+      const unsigned m = __ballot_sync(0xffffffffu, on) & gmask;
+      const int p = n + __popc(m & ((1u << lane) - 1u));
+      n += __popc(m);
+      if (on && p < kCijCand) {
+        ctgt[p] = t;
+        ccode[p] = code;
+        cw[p] = w;
+      }
+    };
+    put(f1 > 0.0, k1, f1, 1u << 15 | (unsigned)gl << 10);
+    for (int r = 0; r < rounds; r++) {
+      // this lane's 2-bond path: slot e of the s1-th partner
+      int e = r * kCijGroup + gl, s1 = -1;
+      for (int s = 0; s < kCijGroup; s++) {
+        const int ns = __shfl_sync(0xffffffffu, n1, gbase + s);
+        if (s1 < 0) {
+          if (e < ns) s1 = s;
+          else e -= ns;
+        }
+      }
+      const int k = __shfl_sync(0xffffffffu, k1, gbase + (s1 & (kCijGroup - 1)));
+      double f12 = __shfl_sync(0xffffffffu, f1, gbase + (s1 & (kCijGroup - 1)));
+      int m = -1, nb3 = 0;
+      if (s1 >= 0) {
+        m = B.bj[k * B.mb + e];
+        f12 *= B.bu[k * B.mb + e].w;
+        if (m != a) nb3 = B.nb[m];
+      }
+      const bool on = nb3 > 0 && f12 > 0.0;
+      const unsigned c12 = (unsigned)s1 << 10 | (unsigned)e << 5;
+      put(on, m, f12, 2u << 15 | c12);
+      const int most = __reduce_max_sync(0xffffffffu, nb3);
+      for (int s3 = 0; s3 < most; s3++) {
+        int t = a;
+        double w = 0.0;
+        if (on && s3 < nb3) {
+          t = B.bj[m * B.mb + s3];
+          w = f12 * B.bu[m * B.mb + s3].w;
+        }
+        put(t != a && t != k && w > 0.0, t, w, 3u << 15 | c12 | (unsigned)s3);
+      }
+    }
+    wide = wide || n > kCijCand;
+    if (wide) n = 0;
+    // the targets are read four at a time
+    if (gl < ((4 - (n & 3)) & 3)) ctgt[n + gl] = kCijNone;
+    __syncwarp();
+    unsigned lost = 0u;  // bit r: this lane's r-th candidate is beaten
+    for (int r = 0, c = gl; c < n; r++, c += kCijGroup) {
+      const int t = ctgt[c];
+      unsigned long long same[2] = {0ull, 0ull};
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        for (int v = 64 * h; v < min(n, 64 * h + 64); v += 4) {
+          const int4 x = *reinterpret_cast<const int4*>(ctgt + v);
+          const unsigned s = (x.x == t) | (x.y == t) << 1 | (x.z == t) << 2 | (x.w == t) << 3;
+          same[h] |= (unsigned long long)s << (v & 63);
+        }
+      same[c >> 6] &= ~(1ull << (c & 63));
+      if ((same[0] | same[1]) == 0ull) continue;
+      const double w = cw[c];
+      const unsigned code = ccode[c];
+#pragma unroll
+      for (int h = 0; h < 2; h++)
+        while (same[h]) {
+          const int j = 64 * h + __ffsll((long long)same[h]) - 1;
+          same[h] &= same[h] - 1;
+          const double wj = cw[j];
+          if (wj > w || (wj == w && ccode[j] < code)) lost |= 1u << r;
+        }
+    }
+    __syncwarp();
+    int nent = 0;
+    for (int r = 0, c = gl; c < n; r++, c += kCijGroup) {
+      if (lost >> r & 1u) ctgt[c] = kCijNone;
+      else nent++;
+    }
+    for (int o = kCijGroup / 2; o > 0; o >>= 1) nent += __shfl_xor_sync(0xffffffffu, nent, o);
+    __syncwarp();
+    // (one place is the atom's own entry, which the reference's table holds)
+    if (nent > T.cap - 1) {
+      wide = true;
+      n = 0;
+    }
+    unsigned mlo = 0u, mhi = 0u;
+    for (int r = 0, c = gl; c < n; r++, c += kCijGroup) {
+      if (lost >> r & 1u) continue;
+      const int t = ctgt[c];
+      int rank = 0;
+      for (int v = 0; v < n; v += 4) {
+        const int4 x = *reinterpret_cast<const int4*>(ctgt + v);
+        rank += (x.x < t) + (x.y < t) + (x.z < t) + (x.w < t);
+      }
+      const unsigned code = ccode[c];
+      const int len = (int)(code >> 15);
+      int k = -1, m = -1;
+      if (len > 1) k = B.bj[q1 + (code >> 10 & 31)];
+      if (len > 2) m = B.bj[k * B.mb + (code >> 5 & 31)];
+      const long o = (long)a * T.cap + rank;
+      T.ent[o] = make_int4(t, len, k, m);
+      T.w[o] = cw[c];
+      if (t & 32) mhi |= 1u << (t & 31);
+      else mlo |= 1u << (t & 31);
+    }
+    for (int o = kCijGroup / 2; o > 0; o >>= 1) {
+      mlo |= __shfl_xor_sync(0xffffffffu, mlo, o);
+      mhi |= __shfl_xor_sync(0xffffffffu, mhi, o);
+    }
+    if (live && gl == 0) {
+      if (wide) {
+        cij_build_atom<kCijLocal>(B, T, a, status);
+      } else {
+        T.cnt[a] = nent;
+        T.mask[a] = (unsigned long long)mhi << 32 | mlo;
+      }
+    }
+    __syncwarp();  // this atom's candidates are read before the next one's are laid down
+  }
 }
 
 // The LJ list's near sublist: the entries within R2 + kLjNearSkin of the
@@ -1425,6 +1589,8 @@ struct mdg_ctx {
 
   unsigned int* d_status = nullptr;
   int special_blocks = 0;
+  int cij_blocks = 0;         // resident blocks of the connectivity kernel (grid-stride over atoms)
+  int* cij_scratch = nullptr; // its candidates, a row per resident group
   int warp_blocks = 0;        // resident blocks of the warp-per-atom LJ list kernels (grid-stride over atoms)
 
   // one MD step captured as a CUDA graph (replayed when no per-step energies are wanted)
@@ -1617,7 +1783,9 @@ void free_system(mdg_ctx* c)
   }
   void* lq[] = {c->cij.cnt, c->cij.ent, c->cij.w, c->cij.mask, c->spc.cnt, c->spc.part, c->spc.off,
                 c->spc.flat, c->spc.trec, c->spc.rec, c->spc.mid, c->spc.midc, c->spc.work,
-                c->spc.ctr, c->lj_inr, c->lj_inr_cnt, c->ljt.cnt, c->ljt.list, c->ljt.pos0};
+                c->spc.ctr, c->lj_inr, c->lj_inr_cnt, c->ljt.cnt, c->ljt.list, c->ljt.pos0,
+                c->cij_scratch};
+  c->cij_scratch = nullptr;
   std::memset(&c->ljt, 0, sizeof(NList));
   c->lj_inr = nullptr;
   c->lj_inr_cnt = nullptr;
@@ -1960,7 +2128,8 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
   if (pot & MDG_POT_BRENNER)
     LAUNCH(c, "brenner", k_brenner, nblk(c->n), kThreads, c->d_bp, c->d_btables, B, c->fo, c->d_status);
   if (lj) {
-    LAUNCH(c, "cij_table", k_cij, nblk(c->n), kThreads, B, c->cij, c->spc.ctr, c->d_status);
+    LAUNCH(c, "cij_table", k_cij, std::min(nblk(c->n, kCijAtoms), c->cij_blocks), kCijThreads, B, c->cij,
+           c->cij_scratch, c->spc.ctr, c->d_status);
     if (ovl) CK(cudaStreamWaitEvent(c->stream, c->ev_join2, 0));
     const int pairs = (c->bt.ctr && c->bt.pairs) ? 1 : 0;
     const int lgrid = nblk(c->n * kLjGroup, kLjThreads);
@@ -2468,6 +2637,11 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_lj_filter, kThreads, 0);
     c->warp_blocks = sms * (per > 0 ? per : 1);
+    per = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_cij, kCijThreads, 0);
+    c->cij_blocks = std::min(nblk(n, kCijAtoms), sms * (per > 0 ? per : 1));
+    c->cij_scratch = dalloc<int>((size_t)c->cij_blocks * kCijAtoms * kCijScratch);
+    if (!c->cij_scratch) return fail(MDG_ERR_CUDA, "cudaMalloc (connectivity)");
   }
   if (cudaHostAlloc((void**)&c->h_stage, 2 * (size_t)n * sizeof(double4), cudaHostAllocDefault) != cudaSuccess)
     return fail(MDG_ERR_CUDA, "cudaHostAlloc (staging)");
