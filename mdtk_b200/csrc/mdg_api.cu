@@ -638,6 +638,107 @@ __global__ void k_brenner(const BrennerParams* P, const BrennerTables* T, BondLi
   brenner_atom(R, O, a);
 }
 
+// b-bar of a Brenner bond (i, j), i < j, p = i -> j (Brenner::baver), on the
+// bond's lane pair: lane e evaluates B of its own end (i for e = 0, j for
+// e = 1) with its gradient and its end's part of F's; F itself, a value of both
+// ends' coordinations, is evaluated by both lanes.
+__device__ double brenner_baver_end(const Brenner& R, int e, int i, int j, const PairG& p, double V,
+                                    EndSinkT<double>& sink, unsigned pm)
+{
+  const PairG q = pair_reverse(p);
+  const int me = e ? j : i, ot = e ? i : j;
+  const double bmine = R.Bterm(me, ot, e ? q : p, V / 2.0, sink);
+  const double bother = pair_swap(bmine, pm);
+  double val = (bmine + bother) / 2.0;
+  if (R.type(i) != kC || R.type(j) != kC) return val;
+  Sink dummy;
+  const double Nti = R.Nsum(i, j, 0, 0.0, dummy), Ntj = R.Nsum(j, i, 0, 0.0, dummy);
+  const double Nc = R.nconj(i, j, 0.0, dummy);
+  double F[4];
+  f_eval(R.T, Nti, Ntj, Nc, F, R.status);
+  val += F[0] / 2.0;
+  if (V != 0.0) {
+    const double Vh = V / 2.0;
+    R.Nsum(me, ot, 0, F[e ? 2 : 1] * Vh, sink);
+    double acc = 0.0;
+    R.nconj_side(me, ot, acc, F[3] * Vh, sink);
+  }
+  return val;
+}
+
+// Brenner on lane pairs, as rebo_end_task: lane e writes the record of its end
+// of the bond; lane 0 adds the pair terms and the bond's energy.
+__device__ void brenner_end_task(const Brenner& R, double* rec, int e, int lo, int s, int hi)
+{
+  const BondList& B = R.B;
+  const unsigned pm = 3u << ((threadIdx.x & 31) & ~1);
+  const int nbm = B.nb[e ? hi : lo];
+  EndSinkT<double> sink;
+  sink.me = e ? hi : lo;
+  sink.lo = lo;
+  sink.hi = hi;
+  sink.pair_on = true;
+  sink.glo = v3(0, 0, 0);
+  sink.ghi = v3(0, 0, 0);
+  sink.A = rec + 5;
+  sink.W = rec + 5 + 3 * nbm;
+  for (int t = 0; t < 4 * nbm; t++) sink.A[t] = 0.0;
+  const PairG p = pair_from_slot(B, lo * B.mb + s);
+  Sink dummy;
+  const double vav = R.Vexp(lo, hi, p, true, 0.0, dummy);
+  double E = R.Vexp(lo, hi, p, false, e == 0 ? 1.0 : 0.0, sink);
+  if (vav != 0.0) {
+    const double bav = brenner_baver_end(R, e, lo, hi, p, -vav, sink, pm);
+    E += -bav * R.Vexp(lo, hi, p, true, e == 0 ? -bav : 0.0, sink);
+  }
+  const double ox = __shfl_xor_sync(pm, e ? sink.glo.x : sink.ghi.x, 1);
+  const double oy = __shfl_xor_sync(pm, e ? sink.glo.y : sink.ghi.y, 1);
+  const double oz = __shfl_xor_sync(pm, e ? sink.glo.z : sink.ghi.z, 1);
+  const V3 g = e ? sink.ghi : sink.glo;
+  rec[0] = g.x + ox;
+  rec[1] = g.y + oy;
+  rec[2] = g.z + oz;
+  rec[3] = e ? 0.0 : E;
+  rec[4] = 0.0;
+}
+
+// Brenner (and torsion) by bond ends on lane pairs, the torsion of each C-C
+// bond an item of its own: the items of k_rebo_split_task.  Bound by the
+// serial chain of one end: a thread per atom walked all of an atom's bonds,
+// both ends of each (1,000 diamond atoms: 207 us; so 36 us).
+__global__ void __launch_bounds__(128) k_brenner_split_task(const BrennerParams* P, const BrennerTables* T,
+                                                            const ReboParams* RP, const ReboTables* RT, BondList B,
+                                                            TorsParams TP, int do_tors, BondTasks K,
+                                                            unsigned int* status)
+{
+  pdl_enter();
+  const long n0 = (long)K.ctr[0], n1 = (long)K.ctr[1];
+  const long ntor = do_tors ? n0 : 0;
+  const long base1 = (2 * n0 + ntor + 1) & ~1L;
+  const long total = base1 + 2 * n1;
+  Brenner R{*P, *T, B, status};
+  Rebo RR{*RP, *RT, B, status};  // the torsion term's types and bonds
+  const long stride = (long)gridDim.x * blockDim.x, t0 = spread_task_index();
+  for (long t = t0; t < total; t += stride) {  // (stride and total are even: both lanes of a pair stay together)
+    const bool cc_end = t < 2 * n0, tors = !cc_end && t < 2 * n0 + ntor;
+    if (!cc_end && !tors && t < base1) continue;  // the padding item
+    const long b = cc_end ? (t >> 1) : (tors ? t - 2 * n0 : ((t - base1) >> 1));
+    const int q = (cc_end || tors) ? K.q[b] : K.q[K.cap - 1 - b];
+    const int lo = q / B.mb, s = q - lo * B.mb;
+    const int hi = B.bj[q], sh = B.brev[q];
+    const long rl = K.rbase[lo], rh = K.rbase[hi];
+    if (rl < 0 || rh < 0 || sh < 0) continue;  // already flagged
+    const int rsl = bond_rec_size(B.nb[lo]), rsh = bond_rec_size(B.nb[hi]);
+    if (tors) {
+      rebo_tors_task(RR, TP, K.rec + rl + (long)(B.nb[lo] + cc_index(B, lo, s)) * rsl,
+                     K.rec + rh + (long)(B.nb[hi] + cc_index(B, hi, sh)) * rsh, lo, s, hi);
+    } else {
+      const int e = (int)(t & 1);
+      brenner_end_task(R, e ? K.rec + rh + (long)sh * rsh : K.rec + rl + (long)s * rsl, e, lo, s, hi);
+    }
+  }
+}
+
 constexpr int kCijLocal = 128;  // per-thread connectivity table capacity
 
 // Connectivity tables, kCijGroup lanes per atom: cij_build_atom's entries by
@@ -1981,6 +2082,7 @@ inline void launch_kernel(bool pdl, cudaStream_t st, void (*k)(P...), dim3 grid,
 // when a step is given; before it, the bath temperature) in one pass over
 // the atoms.
 constexpr int kDispParts = 592;  // 4 blocks per SM of a B200: at most one atom per thread on the liquid
+constexpr double kBrennerRecBytes = 8e9;  // Brenner's bond records: 0.9 M atoms at 16 bonds an atom
 constexpr int kMetalListCap = 320;  // metal / ion list partners per atom (fcc Cu holds ~180 within 7.92 A)
 constexpr int kBathBlocks = 120;
 int step_start(mdg_ctx* c, const StepDev* step)
@@ -2086,7 +2188,10 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
     rs = c->side;
   }
   LAUNCH_ON(c, rs, "bonds_rev", k_brev, nblk(c->n), kThreads, c->bb, c->bt, c->d_status);
-  if (tasks) {
+  if (tasks && (pot & MDG_POT_BRENNER)) {
+    LAUNCH(c, "brenner", k_brenner_split_task, c->rebo_task_blocks, kThreads, c->d_bp, c->d_btables, c->d_rp,
+           c->d_tables, B, c->tp, tors ? 1 : 0, c->bt, c->d_status);
+  } else if (tasks) {
     const int ir = rebo ? 1 : 0, it = tors ? 1 : 0;
     const int grid = c->rebo_grid > 0 ? c->rebo_grid : c->rebo_task_blocks;
     if (f32p && c->bt.pairs == 2) {
@@ -2125,7 +2230,7 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
               c->spc, 0, c->fo);
     CK(cudaEventRecord(c->ev_join, c->side));
   }
-  if (pot & MDG_POT_BRENNER)
+  if (!tasks && (pot & MDG_POT_BRENNER))
     LAUNCH(c, "brenner", k_brenner, nblk(c->n), kThreads, c->d_bp, c->d_btables, B, c->fo, c->d_status);
   if (lj) {
     LAUNCH(c, "cij_table", k_cij, std::min(nblk(c->n, kCijAtoms), c->cij_blocks), kCijThreads, B, c->cij,
@@ -2580,12 +2685,19 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     return fail(MDG_ERR_CUDA, "cudaMalloc (bonds)");
   CK(cudaMemset(c->fo.glj, 0, n * sizeof(double4)));
   CK(cudaMemset(c->fo.e_lj, 0, n * sizeof(double)));
-  if (c->prm.potentials & (MDG_POT_REBO | MDG_POT_ETORS) && !(c->prm.potentials & MDG_POT_BRENNER)) {
+  // Brenner's records are sized for atoms with every bond slot in use (its
+  // per-atom kernel has no such limit); beyond kBrennerRecBytes that kernel is
+  // taken instead.
+  const bool brenner = c->prm.potentials & MDG_POT_BRENNER;
+  const int tors1 = (c->prm.potentials & MDG_POT_ETORS) ? 1 : 0;
+  const double brenner_rec = (double)n * mb * (1 + tors1) * bond_rec_size(mb);
+  if (brenner ? brenner_rec * sizeof(double) <= kBrennerRecBytes
+              : (c->prm.potentials & (MDG_POT_REBO | MDG_POT_ETORS)) != 0) {
     BondTasks& K = c->bt;
     K.cap = n * mb;
-    K.pairs = c->prm.task_mode >= 2 ? c->prm.task_mode - 1 : 0;
-    K.tors = (c->prm.potentials & MDG_POT_ETORS) ? 1 : 0;
-    K.rec_cap = (long)n * c->prm.bond_rec_avg;
+    K.pairs = brenner ? 2 : (c->prm.task_mode >= 2 ? c->prm.task_mode - 1 : 0);
+    K.tors = tors1;
+    K.rec_cap = brenner ? (long)brenner_rec : (long)n * c->prm.bond_rec_avg;
     K.q = dalloc<int>((size_t)K.cap);
     K.ctr = dalloc<unsigned long long>(4);
     K.rbase = dalloc<long>(n);
@@ -2598,6 +2710,8 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (c->prm.precision == MDG_PREC_FP32_MIXED)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rebo_task<f32, ReboTables32>, kThreads, 0);
+    else if (brenner)
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_brenner_split_task, kThreads, 0);
     else
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_rebo_task<double, ReboTables>, kThreads, 0);
     c->rebo_task_blocks = sms * (per > 0 ? per : 1);
@@ -2879,6 +2993,7 @@ static int autotune(mdg_ctx* c)
 {
   if (c->tuned || !c->bt.ctr) return MDG_OK;
   c->tuned = true;
+  if (c->prm.potentials & MDG_POT_BRENNER) return MDG_OK;  // one split, no LJ chain to overlap with
   const bool lj = c->prm.potentials & MDG_POT_AIREBO_LJ;
   // a fixed task mode (task_mode 1 or 2) keeps its split; the launch
   // configuration, which never changes results, is still chosen
@@ -3270,7 +3385,7 @@ int mdg_tuned_launch(mdg_ctx* c, int* overlap, int* rebo_blocks)
 {
   if (!c) return fail(MDG_ERR_ARG, "null context");
   if (overlap) *overlap = c->overlap ? 1 : 0;
-  if (rebo_blocks) *rebo_blocks = c->rebo_grid > 0 ? c->rebo_grid : c->rebo_task_blocks;
+  if (rebo_blocks) *rebo_blocks = (c->prm.potentials & MDG_POT_BRENNER) ? 0 : c->rebo_grid > 0 ? c->rebo_grid : c->rebo_task_blocks;
   return MDG_OK;
 }
 
@@ -3285,7 +3400,7 @@ int mdg_set_dependent_launch(mdg_ctx* c, int on)
 int mdg_task_mode(mdg_ctx* c, int* mode, float* ms_directed, float* ms_per_bond, float* ms_split)
 {
   if (!c) return fail(MDG_ERR_ARG, "null context");
-  if (mode) *mode = c->bt.pairs + 1;
+  if (mode) *mode = (c->prm.potentials & MDG_POT_BRENNER) ? 1 : c->bt.pairs + 1;  // (the REBO splits)
   if (ms_directed) *ms_directed = c->tune_ms[0];
   if (ms_per_bond) *ms_per_bond = c->tune_ms[1];
   if (ms_split) *ms_split = c->tune_ms[2];

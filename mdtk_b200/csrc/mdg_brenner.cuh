@@ -189,11 +189,10 @@ struct Brenner {
       double ex = 1.0;
       if (al != 0.0) ex = exp(al * ((p.r - P.Re[tc][to]) - (rv.w - P.Re[tc][tk])));
       if (ex == 0.0) continue;
-      Sink dummy;
-      double gv = G(c, o, p, s, brv, rv.w, bu3, 0.0, dummy);
+      // one evaluation: the value G returns does not depend on the seed
       double fv = u.w;
+      double gv = G(c, o, p, s, brv, rv.w, bu3, fv * ex * V, sink);
       if (V != 0.0) {
-        G(c, o, p, s, brv, rv.w, bu3, fv * ex * V, sink);
         double df = B.bd[q].x;
         if (df != 0.0) sink.cbond(c, s, bu3 * ((gv * ex * V) * df));
         if (al != 0.0) {
@@ -218,11 +217,12 @@ struct Brenner {
     Sink dummy;
     double DVal = D(c, o, p, 0.0, dummy);
     const double dl = P.delta[type(c)][type(c)];
+    const double val = pow(DVal, -dl);
     if (V != 0.0) {
-      double Der = -dl * pow(DVal, -dl - 1.0);
+      double Der = -dl * (val / DVal);  // -dl D^(-dl-1)
       D(c, o, p, Der * V, sink);
     }
-    return pow(DVal, -dl);
+    return val;
   }
 
   // N_conj (Brenner::Nconj, Brenner.cxx:353-413): 1 + sum_k f_ck F(N_kc) + sum_l f_ol F(N_lo).
