@@ -493,8 +493,7 @@ int mdg_set_param(mdg_ctx* c, int id, double value)
   CK(cudaStreamSynchronize(c->stream));
   // forces changed: the captured step (kernel arguments hold the LJ
   // parameters) and the stored accelerations are stale
-  if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
-  c->step_graph = nullptr;
+  drop_step_graphs(c);
   c->acc_valid = false;
   if (c->adj) c->adj->have_fwd = false;
   return MDG_OK;
@@ -585,7 +584,7 @@ int mdg_adjoint_forward(mdg_ctx* c, int nsteps, double dt, int every, double* po
     if (!rc && s % every == 0 && s < nsteps) rc = adj_save(c, s / every);
   }
   if (rc) return rc;
-  rc = reduce_energies(c, c->d_energy, 0, 0, true);
+  rc = reduce_energies(c, c->d_energy, nullptr, true);
   if (rc) return rc;
   rc = d2d(c, w->fin_pos, c->pos, n);
   if (!rc) rc = d2d(c, w->fin_vel, c->vel, n);

@@ -43,7 +43,7 @@ int fail(int code, const std::string& msg)
   } while (0)
 
 constexpr int kThreads = 128;
-constexpr int kRedBlocks = 120;
+constexpr int kRedBlocks = 296;  // two per SM
 constexpr double kAo = 1e-8, kEv = 1.6021e-12, kFs = 1e-15;
 
 inline int nblk(int n, int t = kThreads) { return (n + t - 1) / t; }
@@ -1481,51 +1481,90 @@ __global__ void k_ekin(State S, double* ekin)
   ekin[i] = S.mass[i] * (v.x * v.x + v.y * v.y + v.z * v.z) / 2.0 / kAccConv;
 }
 
-// Deterministic sums of up to 4 per-atom arrays: fixed grid, fixed order.
+// Deterministic sums of up to 5 per-atom arrays in one pass: each block sums
+// its strided share of every array, and the last block to finish (a counter,
+// no waiting) adds the blocks' partials in a fixed order, a warp per array.
+// Bound by latency: two launches, the second a chain of 120 additions on one
+// thread per sum, took 17 us a step beside a 1,728-atom diamond's 76; so 4.
 struct RedArgs {
   const double* a[5];
   int slot[5];  // output slot of each array (the metal energies join another slot or take their own)
   int narr, nout, n;
 };
-__global__ void k_reduce_partial(RedArgs R, double* part)
+// out row of the sums: row *ctr when ctr is given (the step log's row, counted
+// up by the last block), else row 0.  grad (or null) is checked for
+// non-finite values on the way.
+__global__ void __launch_bounds__(kThreads) k_energy_sum(RedArgs R, const double4* grad, double* part,
+                                                         unsigned int* done, double* out, int stride, int* ctr,
+                                                         unsigned int* status)
 {
   pdl_enter();
-  __shared__ double sh[kThreads];
-  int which = blockIdx.y;
-  const double* x = R.a[which];
-  double s = 0.0;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < R.n; i += gridDim.x * blockDim.x) s += x[i];
-  sh[threadIdx.x] = s;
+  __shared__ double sh[5][kThreads / 32];
+  __shared__ int last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, i0 = blockIdx.x * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int k = 0; k < 5; k++) {  // (unrolled: R.a stays in the parameters)
+    if (k >= R.narr) break;
+    const double* x = R.a[k];
+    double s = 0.0;
+    for (int i = i0; i < R.n; i += gridDim.x * blockDim.x) s += x[i];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) sh[k][wid] = s;
+  }
+  if (grad) {
+    bool bad = false;
+    for (int i = i0; i < R.n; i += gridDim.x * blockDim.x) {
+      const double4 v = grad[i];
+      bad |= !isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z);
+    }
+    if (bad) atomicOr(status, ST_NONFINITE);
+  }
   __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
+  if (threadIdx.x < R.narr) {
+    double s = 0.0;
+    for (int w = 0; w < kThreads / 32; w++) s += sh[threadIdx.x][w];
+    part[threadIdx.x * gridDim.x + blockIdx.x] = s;
   }
-  if (threadIdx.x == 0) part[which * gridDim.x + blockIdx.x] = sh[0];
-}
-// out[w] = sum of the partials of the arrays of slot w (in array order)
-__global__ void k_reduce_final(const double* part, int nparts, RedArgs R, double* out, int slot_stride, int slot,
-                               unsigned int* status)
-{
-  pdl_enter();
-  int w = threadIdx.x;
-  if (w >= R.nout) return;
-  double s = 0.0;
-  for (int k = 0; k < R.narr; k++) {
-    if (R.slot[k] != w) continue;
-    double t = 0.0;
-    for (int q = 0; q < nparts; q++) t += part[k * nparts + q];
-    s = (k == w) ? t : s + t;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int k = wid; k < R.narr; k += kThreads / 32) {
+    double s = 0.0;
+    for (int q = lane; q < (int)gridDim.x; q += 32) s += __ldcg(part + k * gridDim.x + q);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) sh[k][0] = s;
   }
-  out[slot * slot_stride + w] = s;
-  if (!isfinite(s)) atomicOr(status, ST_NONFINITE);
+  __syncthreads();
+  const int row = ctr ? *ctr : 0;
+  __syncthreads();
+  if (threadIdx.x < R.nout) {
+    // the arrays of this slot, in array order
+    double s = 0.0;
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      if (k >= R.narr || R.slot[k] != (int)threadIdx.x) continue;
+      s = k == (int)threadIdx.x ? sh[k][0] : s + sh[k][0];
+    }
+    out[(long)row * stride + threadIdx.x] = s;
+    if (!isfinite(s)) atomicOr(status, ST_NONFINITE);
+  }
+  if (threadIdx.x == 0) {
+    if (ctr) *ctr = row + 1;
+    *done = 0u;
+  }
 }
 
 // Per-system energy sums of a batched context: one block per system; each
 // thread sums a strided share of the system's atoms, then a fixed tree
 // (deterministic).  out[4 s + {0,1,2,3}] = REBO, LJ, torsion, kinetic.
+// out row *ctr when ctr is given (rows of 4 gridDim.x, counted up by the last
+// block to finish), else row 0.
 __global__ void k_sys_energy(const int64_t* first, int64_t n, const double* er, const double* el, const double* et,
-                             const double* ek, const double* em, double* out, unsigned int* status)
+                             const double* ek, const double* em, double* out, int* ctr, unsigned int* done,
+                             unsigned int* status)
 {
   pdl_enter();
   __shared__ double sh[4][kThreads];
@@ -1547,20 +1586,18 @@ __global__ void k_sys_energy(const int64_t* first, int64_t n, const double* er, 
       for (int q = 0; q < 4; q++) sh[q][threadIdx.x] += sh[q][threadIdx.x + w];
     __syncthreads();
   }
+  const long row = ctr ? *ctr : 0;
   if (threadIdx.x < 4) {
     const double v = sh[threadIdx.x][0];
-    out[4 * sy + threadIdx.x] = v;
+    out[4 * (row * gridDim.x + sy) + threadIdx.x] = v;
     if (!isfinite(v)) atomicOr(status, ST_NONFINITE);
   }
-}
-
-__global__ void k_finite(const double4* g, int n, unsigned int* status)
-{
-  pdl_enter();
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double4 v = g[i];
-  if (!isfinite(v.x) || !isfinite(v.y) || !isfinite(v.z)) atomicOr(status, ST_NONFINITE);
+  if (!ctr) return;
+  __syncthreads();  // every thread has read the row
+  if (threadIdx.x == 0 && atomicAdd(done, 1u) == gridDim.x - 1) {
+    *ctr = (int)row + 1;
+    *done = 0u;
+  }
 }
 
 // FMA-throughput probes for the roofline denominators (no peak for the FP64
@@ -1606,6 +1643,16 @@ namespace {
 struct AdjWs;  // adjoint-path buffers (mdg_adjoint.cuh)
 }
 
+// One MD step captured as a CUDA graph, and what it was captured with.
+struct StepGraph {
+  cudaGraphExec_t exec = nullptr;
+  double dt = 0.0;
+  int cfg = -1;                   // step_cfg
+  const double* elog = nullptr;   // the energy log it writes
+  cudaStream_t stream = nullptr;
+  int launches = 0;
+};
+
 struct mdg_ctx {
   mdg_params prm;
   ReboParams rp;
@@ -1648,7 +1695,8 @@ struct mdg_ctx {
   Grid grid[3];
   int* d_need = nullptr;   // [4]: lists 0-2, the LJ near sublist
   int* d_force = nullptr;  // [4]
-  unsigned int* d_disp_done = nullptr;  // blocks of step_start finished (back to 0 by the last)
+  unsigned int* d_disp_done = nullptr;  // blocks finished of step_start, the energy sums (back to 0 by the last)
+                                        // and, third, the row of the step log
   double* d_part = nullptr;
   double rcut[3] = {0, 0, 0};
   bool has_list[3] = {false, false, false};
@@ -1694,10 +1742,9 @@ struct mdg_ctx {
   int* cij_scratch = nullptr; // its candidates, a row per resident group
   int warp_blocks = 0;        // resident blocks of the warp-per-atom LJ list kernels (grid-stride over atoms)
 
-  // one MD step captured as a CUDA graph (replayed when no per-step energies are wanted)
-  cudaGraphExec_t step_graph = nullptr;
-  double graph_dt = 0.0;
-  int graph_cfg = -1;           // step_cfg the graph was captured with
+  // captured steps by what they log (step_and_log): nothing, the total
+  // energies, each system's
+  StepGraph step_graph[3];
   bool pdl = true;              // programmatic dependent launches (mdg_set_dependent_launch)
   int step_cfg = 0;             // bumped when the thermal bath or the dt mode changes
 
@@ -1716,8 +1763,6 @@ struct mdg_ctx {
   double* d_time = nullptr;             // [nsys] simulated time since the mode was set
   unsigned long long* d_vmax = nullptr; // [nsys] bits of the step's largest |v|
   double* d_dt_prev = nullptr;          // [nsys] the step just taken (SimLoop::dt_prev)
-  cudaStream_t graph_stream = nullptr;
-  int graph_launches = 0;
 
   // SimLoop bookkeeping kept for the checkpoint and trajectory files
   // (SimLoopSaver, SimLoop::saveToStreamXVA): the iteration counter, the time
@@ -1840,6 +1885,14 @@ int status_to_code(unsigned int st, std::string& msg)
   return code;
 }
 
+void drop_step_graphs(mdg_ctx* c)
+{
+  for (StepGraph& g : c->step_graph) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+  }
+}
+
 void adj_free(mdg_ctx* c);
 void io_release(mdg_ctx* c);
 void io_free(mdg_ctx* c);
@@ -1890,8 +1943,7 @@ void free_system(mdg_ctx* c)
   std::memset(&c->ljt, 0, sizeof(NList));
   c->lj_inr = nullptr;
   c->lj_inr_cnt = nullptr;
-  if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
-  c->step_graph = nullptr;
+  drop_step_graphs(c);
   for (void* p : lq)
     if (p) cudaFree(p);
   std::memset(&c->cij, 0, sizeof(c->cij));
@@ -2285,7 +2337,10 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
 
 // Sums of rebo, lj, tors (, kin) into slots 0-3; the metal and ion energies
 // join the torsion slot, or take slot 3 of their own (split_metal, no kin).
-int reduce_energies(mdg_ctx* c, double* out_dev, int slot_stride, int slot, bool with_kin, bool split_metal = false)
+// log_row: device counter of the step log's row (null: out_dev itself); grad:
+// also check it for non-finite values.
+int reduce_energies(mdg_ctx* c, double* out_dev, int* log_row, bool with_kin, bool split_metal = false,
+                    const double4* grad = nullptr)
 {
   RedArgs R;
   R.a[0] = c->fo.e_rebo;
@@ -2302,9 +2357,8 @@ int reduce_energies(mdg_ctx* c, double* out_dev, int slot_stride, int slot, bool
     if (split_metal && !with_kin) R.nout = 4;
   }
   R.n = c->n;
-  LAUNCH(c, "energy_partial", k_reduce_partial, dim3(kRedBlocks, R.narr), kThreads, R, c->d_red_part);
-  LAUNCH(c, "energy_final", k_reduce_final, 1, 32, c->d_red_part, kRedBlocks, R, out_dev, slot_stride, slot,
-         c->d_status);
+  LAUNCH(c, "energy_sum", k_energy_sum, std::min(nblk(c->n), kRedBlocks), kThreads, R, grad, c->d_red_part,
+         c->d_disp_done + 1, out_dev, 4, log_row, c->d_status);
   return launch_check(c);
 }
 
@@ -2429,7 +2483,7 @@ int mdg_create(const mdg_params* p, mdg_ctx** out)
   c->d_status = dalloc<unsigned int>(1);
   c->d_need = dalloc<int>(4);
   c->d_force = dalloc<int>(4);
-  c->d_disp_done = dalloc<unsigned int>(1);
+  c->d_disp_done = dalloc<unsigned int>(4);
   c->d_energy = dalloc<double>(8);
   if (!c->d_status || !c->d_need || !c->d_force || !c->d_disp_done || !c->d_energy) {
     mdg_destroy(c);
@@ -2438,7 +2492,7 @@ int mdg_create(const mdg_params* p, mdg_ctx** out)
   cudaMemset(c->d_status, 0, sizeof(unsigned int));
   cudaMemset(c->d_need, 0, 4 * sizeof(int));
   cudaMemset(c->d_force, 0, 4 * sizeof(int));
-  cudaMemset(c->d_disp_done, 0, sizeof(unsigned int));
+  cudaMemset(c->d_disp_done, 0, 4 * sizeof(unsigned int));
   if (cudaGetLastError() != cudaSuccess) { mdg_destroy(c); return fail(MDG_ERR_CUDA, "setup copies failed"); }
   *out = c;
   return MDG_OK;
@@ -2866,9 +2920,8 @@ int mdg_compute(mdg_ctx* c, double* e_total, double* e_terms, double* grad)
   if (!c || !c->n) return fail(MDG_ERR_STATE, "no system loaded");
   int rc = evaluate(c);
   if (rc) return rc;
-  rc = reduce_energies(c, c->d_energy, 0, 0, false, true);
+  rc = reduce_energies(c, c->d_energy, nullptr, false, true, c->grad);
   if (rc) return rc;
-  LAUNCH(c, "finite_check", k_finite, nblk(c->n), kThreads, c->grad, c->n, c->d_status);
   double he[4] = {0, 0, 0, 0};
   CK(cudaMemcpyAsync(he, c->d_energy, (c->has_list[2] ? 4 : 3) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   std::vector<double4> hg;
@@ -3082,32 +3135,46 @@ static StepDev step_dev(mdg_ctx* c, double dtf)
   return P;
 }
 
-static int ensure_step_graph(mdg_ctx* c, double dtf)
+int sys_energies(mdg_ctx* c, double* out_dev, int* log_row);
+
+// log: 0 none, 1 the step's total energies, 2 each system's, into the next
+// row of d_elog.
+static int step_and_log(mdg_ctx* c, double dtf, int log)
 {
-  if (c->step_graph && c->graph_dt == dtf && c->graph_stream == c->stream && c->graph_cfg == c->step_cfg)
+  const StepDev sd = step_dev(c, dtf);
+  int rc = evaluate(c, &sd);  // position update, forces, velocity update
+  if (rc || !log) return rc;
+  int* row = reinterpret_cast<int*>(c->d_disp_done + 2);
+  return log == 1 ? reduce_energies(c, c->d_elog, row, true) : sys_energies(c, c->d_elog, row);
+}
+
+static int ensure_step_graph(mdg_ctx* c, double dtf, int log)
+{
+  StepGraph& G = c->step_graph[log];
+  if (G.exec && G.dt == dtf && (!log || G.elog == c->d_elog) && G.stream == c->stream && G.cfg == c->step_cfg)
     return MDG_OK;
-  if (c->step_graph) cudaGraphExecDestroy(c->step_graph);
-  c->step_graph = nullptr;
+  if (G.exec) cudaGraphExecDestroy(G.exec);
+  G.exec = nullptr;
   cudaGraph_t g = nullptr;
   int64_t l0 = c->launches;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  const StepDev sd = step_dev(c, dtf);
-  int rc = evaluate(c, &sd);
+  int rc = step_and_log(c, dtf, log);
   cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
-  c->graph_launches = (int)(c->launches - l0);
+  G.launches = (int)(c->launches - l0);
   c->launches = l0;
   if (rc) { if (g) cudaGraphDestroy(g); return rc; }
   if (ce != cudaSuccess) return fail(MDG_ERR_CUDA, std::string("stream capture: ") + cudaGetErrorString(ce));
-  ce = cudaGraphInstantiate(&c->step_graph, g, 0);
+  ce = cudaGraphInstantiate(&G.exec, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) return fail(MDG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(ce));
-  c->graph_dt = dtf;
-  c->graph_stream = c->stream;
-  c->graph_cfg = c->step_cfg;
+  G.dt = dtf;
+  G.elog = c->d_elog;
+  G.stream = c->stream;
+  G.cfg = c->step_cfg;
   return MDG_OK;
 }
 
-int sys_energies(mdg_ctx* c, double* out_dev);
+int sys_energies(mdg_ctx* c, double* out_dev, int* log_row);
 // checkpoint and trajectory output around the steps (defined with the file formats)
 int io_run_start(mdg_ctx* c, double dtf, bool fresh);
 int io_before_step(mdg_ctx* c);
@@ -3127,7 +3194,7 @@ static int init_first_step(mdg_ctx* c)
   if (first) {
     LAUNCH(c, "ekin", k_ekin, nblk(c->n), kThreads, S, c->e_kin);
     // one system: the grid-wide reduction (the per-system kernel is one block per system)
-    rc = c->nsys == 1 ? reduce_energies(c, c->d_e0, 0, 0, true) : sys_energies(c, c->d_e0);
+    rc = c->nsys == 1 ? reduce_energies(c, c->d_e0, nullptr, true) : sys_energies(c, c->d_e0, nullptr);
     if (rc) return rc;
     c->e0_dev = true;
     c->chk_eb0 = 0.0;
@@ -3147,8 +3214,47 @@ static void fill_energy_log(mdg_ctx* c, int nsteps, double* epot, double* etot)
   }
 }
 
-// fresh: a new SimLoop::execute (dt_prev = dt); else the continuation of
-// the previous call's loop
+// nsteps steps after init_first_step; log as step_and_log (rows of 4, or 4 per
+// system, from row 0 of d_elog).  fresh: a new SimLoop::execute (dt_prev = dt);
+// else the continuation of the previous call's loop.
+static int step_loop(mdg_ctx* c, int nsteps, double dtf, int log, bool fresh)
+{
+  int rc = io_run_start(c, dtf, fresh);
+  if (rc) return rc;
+  if (log) {
+    const int64_t need = (int64_t)nsteps * 4 * (log == 2 ? c->nsys : 1);
+    if (c->elog_cap < need) {
+      if (c->d_elog) cudaFree(c->d_elog);
+      c->elog_cap = 0;
+      c->d_elog = dalloc<double>((size_t)need);
+      if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
+      c->elog_cap = need;
+    }
+    CK(cudaMemsetAsync(c->d_disp_done + 2, 0, sizeof(int), c->stream));
+  }
+  // Unless profiling, a step and its energy sums are replayed from a CUDA
+  // graph: same kernels, same arguments, no host launch cost.
+  const bool graph = !c->prof && nsteps > 0;
+  if (graph) {
+    rc = ensure_step_graph(c, dtf, log);
+    if (rc) return rc;
+  }
+  for (int s = 0; s < nsteps; s++) {
+    rc = io_before_step(c);  // scheduled state and trajectory files (SimLoop.cxx:263-277)
+    if (rc) return rc;
+    if (graph) {
+      CK(cudaGraphLaunch(c->step_graph[log].exec, c->stream));
+      c->launches += c->step_graph[log].launches;
+    } else {
+      rc = step_and_log(c, dtf, log);
+      if (rc) return rc;
+    }
+    rc = io_after_step(c);
+    if (rc) return rc;
+  }
+  return io_run_end(c);
+}
+
 static int run_steps(mdg_ctx* c, int nsteps, double dt, double* epot, double* etot, bool fresh,
                      bool defer_log = false)
 {
@@ -3161,42 +3267,8 @@ static int run_steps(mdg_ctx* c, int nsteps, double dt, double* epot, double* et
   if (rc) return rc;
   rc = init_first_step(c);
   if (rc) return rc;
-  rc = io_run_start(c, dtf, fresh);
-  if (rc) return rc;
   const bool log = epot || etot;
-  if (log && c->elog_cap < (int64_t)nsteps * 4) {
-    if (c->d_elog) cudaFree(c->d_elog);
-    c->d_elog = dalloc<double>((size_t)nsteps * 4);
-    if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
-    c->elog_cap = (int64_t)nsteps * 4;
-  }
-  // Unless profiling, a step is replayed from a CUDA graph: same kernels,
-  // same arguments, no host launch cost; the per-step energy sums (when
-  // asked for) follow each replay.
-  const bool graph = !c->prof && nsteps > 0;
-  if (graph) {
-    rc = ensure_step_graph(c, dtf);
-    if (rc) return rc;
-  }
-  for (int s = 0; s < nsteps; s++) {
-    rc = io_before_step(c);  // scheduled state and trajectory files (SimLoop.cxx:263-277)
-    if (rc) return rc;
-    if (graph) {
-      CK(cudaGraphLaunch(c->step_graph, c->stream));
-      c->launches += c->graph_launches;
-    } else {
-      const StepDev sd = step_dev(c, dtf);
-      rc = evaluate(c, &sd);  // position update, forces, velocity update
-      if (rc) return rc;
-    }
-    rc = io_after_step(c);
-    if (rc) return rc;
-    if (log) {
-      rc = reduce_energies(c, c->d_elog, 4, s, true);
-      if (rc) return rc;
-    }
-  }
-  rc = io_run_end(c);
+  rc = step_loop(c, nsteps, dtf, log ? 1 : 0, fresh);
   if (rc) return rc;
   if (log) {
     if (c->h_elog_cap < (int64_t)nsteps * 4) {
@@ -3222,10 +3294,10 @@ int mdg_run(mdg_ctx* c, int nsteps, double dt, double* epot, double* etot)
   return run_steps(c, nsteps, dt, epot, etot, true);
 }
 
-int sys_energies(mdg_ctx* c, double* out_dev)
+int sys_energies(mdg_ctx* c, double* out_dev, int* log_row)
 {
   LAUNCH(c, "sys_energy", k_sys_energy, c->nsys, kThreads, c->d_first ? c->d_first : nullptr, (int64_t)c->n, c->fo.e_rebo,
-         c->fo.e_lj, c->fo.e_tors, c->e_kin, c->has_list[2] ? c->d_em : nullptr, out_dev, c->d_status);
+         c->fo.e_lj, c->fo.e_tors, c->e_kin, c->has_list[2] ? c->d_em : nullptr, out_dev, log_row, c->d_disp_done + 3, c->d_status);
   return launch_check(c);
 }
 
@@ -3240,28 +3312,9 @@ int mdg_batch_run(mdg_ctx* c, int nsteps, double dt, double* epot, double* etot)
   if (rc) return rc;
   rc = init_first_step(c);
   if (rc) return rc;
-  rc = io_run_start(c, dtf, true);
+  rc = step_loop(c, nsteps, dtf, 2, true);
   if (rc) return rc;
   const int64_t need = (int64_t)nsteps * c->nsys * 4;
-  if (c->elog_cap < need) {
-    if (c->d_elog) cudaFree(c->d_elog);
-    c->d_elog = dalloc<double>((size_t)need);
-    if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
-    c->elog_cap = need;
-  }
-  for (int s = 0; s < nsteps; s++) {
-    rc = io_before_step(c);
-    if (rc) return rc;
-    const StepDev sd = step_dev(c, dtf);
-    rc = evaluate(c, &sd);  // position update, forces, velocity update
-    if (rc) return rc;
-    rc = io_after_step(c);
-    if (rc) return rc;
-    rc = sys_energies(c, c->d_elog + (int64_t)s * c->nsys * 4);
-    if (rc) return rc;
-  }
-  rc = io_run_end(c);
-  if (rc) return rc;
   std::vector<double> h((size_t)need);
   CK(cudaMemcpyAsync(h.data(), c->d_elog, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
   rc = read_status(c);
@@ -3288,7 +3341,7 @@ int mdg_batch_energies(mdg_ctx* c, double* e_sys)
     if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
     c->elog_cap = (int64_t)c->nsys * 4;
   }
-  rc = sys_energies(c, c->d_elog);
+  rc = sys_energies(c, c->d_elog, nullptr);
   if (rc) return rc;
   std::vector<double> h((size_t)c->nsys * 4);
   CK(cudaMemcpyAsync(h.data(), c->d_elog, h.size() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
