@@ -47,6 +47,8 @@ struct AdjWs {
   dual4 *brv = nullptr, *bu = nullptr, *bd = nullptr, *nco = nullptr;
   dual *A = nullptr, *W = nullptr, *er = nullptr, *et = nullptr, *el = nullptr, *dp = nullptr;
   dual4 *gown = nullptr, *glj = nullptr, *g = nullptr;
+  dual* brec = nullptr;               // bond-slot records (adj_rec_size)
+  long brcap = 0;                     // record doubles of the FP64 path they were sized by
   dual* cw = nullptr;                 // connectivity weights
   dual *trec = nullptr, *tmidc = nullptr, *tdp = nullptr;  // special-pair task records
   int4* tmid = nullptr;
@@ -109,29 +111,98 @@ __global__ void k_adj_bonds(State S, const double4* tan, ReboParams P, BondList 
   D.nco[a] = make_dual4(Nt, NC, NH, dual((double)ta));
 }
 
+// A bond slot's record on the adjoint path: own gradient (3), energies (REBO,
+// torsion), parameter derivatives, A (3 nb), W (nb).  The FP64 path's record
+// ranges (rbase, 5 + 4 nb doubles a slot) at twice the size hold them.
+MDG_HD int adj_rec_size(int nb) { return 5 + kNParam + 4 * nb; }
+
+// REBO + torsion of each directed bond slot on duals, kAdjLanes threads an
+// atom, into the slots' records; k_adj_bond_reduce adds them in slot order.
+// Bound by the serial chain of one bond on duals: a thread per atom walked all
+// of an atom's bonds (1,000 diamond atoms: 599 us; so 173 us).
+constexpr int kAdjLanes = 4;
 __global__ void k_adj_rebo(const ReboParams* P, const ReboTables* T, BondListT<dual> B, TorsParams TP, int do_rebo,
-                           int do_tors, ForceOutT<dual> O, unsigned int* status)
+                           int do_tors, int jt, const long* rbase, dual* rec, unsigned int* status)
 {
   pdl_enter();
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = t / kAdjLanes;
   if (a >= B.n) return;
+  const long rb = rbase[a];
+  if (rb < 0) return;  // beyond the record capacity (already flagged)
   ReboT<dual, ReboTables> R{*P, *T, B, status};
-  rebo_atom<true>(R, TP, do_rebo, do_tors, O, a);
+  const int nb = B.nb[a];
+  for (int s = t % kAdjLanes; s < nb; s += kAdjLanes) {
+    dual* r = rec + 2 * rb + (long)s * adj_rec_size(nb);
+    for (int k = 5; k < adj_rec_size(nb); k++) r[k] = 0.0;
+    SinkT<dual, true> sink;
+    sink.a = a;
+    sink.g = v3r<dual>(0.0, 0.0, 0.0);
+    sink.dp = r + 5;
+    sink.A = r + 5 + kNParam;
+    sink.W = sink.A + 3 * nb;
+    sink.jt = jt;
+    const int q = a * B.mb + s;
+    const int b = B.bj[q];
+    PairGT<dual> p = pair_from_slot<dual>(B, q);
+    int lo = a, hi = b;
+    if (b < a) { lo = b; hi = a; p = pair_reverse(p); }
+    dual er = 0.0, et = 0.0;
+    if (do_rebo) {
+      const dual E = R.bond(lo, hi, p, sink);
+      if (a == lo) er = E;
+    }
+    if (do_tors) {
+      const dual E = etors_bond(R, TP, lo, hi, p, sink);
+      if (a == lo) et = E;
+    }
+    r[0] = sink.g.x;
+    r[1] = sink.g.y;
+    r[2] = sink.g.z;
+    r[3] = er;
+    r[4] = et;
+  }
+}
+
+// Sums of an atom's slot records, in slot order, kReduceLanes lanes an atom.
+__global__ void k_adj_bond_reduce(BondListT<dual> B, const long* rbase, const dual* rec, ForceOutT<dual> O)
+{
+  pdl_enter();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = t / kReduceLanes;
+  if (a >= B.n) return;
+  const int nb = B.nb[a], rs = adj_rec_size(nb);
+  const long rb = rbase[a];
+  for (int e = t % kReduceLanes; e < rs; e += kReduceLanes) {
+    dual* dst;
+    const int k = e - 5 - kNParam;
+    if (e < 3) dst = reinterpret_cast<dual*>(O.gown + a) + e;
+    else if (e == 3) dst = O.e_rebo + a;
+    else if (e == 4) dst = O.e_tors + a;
+    else if (k < 0) dst = O.dp + (long)a * kNParam + (e - 5);
+    else dst = k < 3 * nb ? O.A + (long)a * O.mb * 3 + k : O.W + (long)a * O.mb + (k - 3 * nb);
+    dual acc = 0.0;
+    if (rb >= 0)
+      for (int s = 0; s < nb; s++) acc += rec[2 * rb + (long)s * rs + e];
+    *dst = acc;
+  }
 }
 
 // Connectivity weights with tangents along the FP64 table's arg-max paths
 // (the products in the order cij_build_atom forms them).
+// kReduceLanes lanes an atom, an entry each.
 __global__ void k_adj_cij(BondListT<dual> B, CijTable T, dual* w)
 {
   pdl_enter();
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = t / kReduceLanes;
   if (a >= B.n) return;
   auto fb = [&](int c, int o) -> dual {
     const int s = bond_slot(B, c, o);
     return s >= 0 ? B.bu[c * B.mb + s].w : dual(0.0);
   };
   const int cnt = T.cnt[a];
-  for (int e = 0; e < cnt; e++) {
+  for (int e = t % kReduceLanes; e < cnt; e += kReduceLanes) {
     const int4 en = T.ent[(long)a * T.cap + e];
     dual v;
     if (en.y == 1) v = fb(a, en.x);
@@ -141,31 +212,47 @@ __global__ void k_adj_cij(BondListT<dual> B, CijTable T, dual* w)
   }
 }
 
-// Plain LJ pairs (the FP64 path's classification), one thread per atom; the
-// REBO kernel has already zeroed and filled this atom's parameter slots.
-__global__ void k_adj_lj_plain(LJParams P, CijTableT<dual> T, State S, NList L, const double4* tan,
-                               ForceOutT<dual> O)
+// Plain LJ pairs (the FP64 path's classification) of the in-range far lists
+// the FP64 evaluation at these positions left (a plain pair is a far one), kLjGroup
+// lanes per atom; the REBO kernels have already filled this atom's parameter
+// slots.  One thread an atom over the whole Verlet list took 1.18 ms on 1,000
+// diamond atoms, 512 partners each, most of them out of range; so 38 us.
+__global__ void k_adj_lj_plain(LJParams P, CijTableT<dual> T, State S, int lcap, const int* inr, const int* far_cnt,
+                               const double4* tan, ForceOutT<dual> O)
 {
   pdl_enter();
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= S.n) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gl = t % kLjGroup;
+  const bool live = t / kLjGroup < S.n;  // every lane stays for the butterfly
+  const int a = live ? t / kLjGroup : S.n - 1;
   const double4 pa = S.pos[a];
   const V3 xa = v3(pa.x, pa.y, pa.z);
   const int ta = (int)pa.w;
+  dual dp[kNParam] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
   SinkT<dual, true> sk;
   sk.a = a;
   sk.g = v3r<dual>(0.0, 0.0, 0.0);
   sk.A = nullptr;
   sk.W = nullptr;
-  sk.dp = O.dp + (long)a * kNParam;
+  sk.dp = dp;
   sk.jt = 1;
   dual e = 0.0;
-  const int cnt = L.cnt[a];
-  const int* lst = L.list + (long)a * L.cap;
+  const int nf = live ? far_cnt[a] : 0;
+  const int* row = inr + (long)a * lcap;
   const unsigned long long amask = T.mask[a];
-  for (int s = 0; s < cnt; s++) lj_plain_pair<dual>(P, T, S, a, lst[s], xa, ta, amask, sk, e, tan);
-  O.glj[a] = make_dual4(sk.g.x, sk.g.y, sk.g.z, 0.0);
-  O.e_lj[a] = e;
+  for (int s = gl; s < nf; s += kLjGroup) lj_plain_pair<dual>(P, T, S, a, row[s], xa, ta, amask, sk, e, tan, true);
+  auto sum = [](dual x) {
+    for (int o = kLjGroup / 2; o > 0; o >>= 1)
+      x += dual(__shfl_xor_sync(0xffffffffu, x.v, o), __shfl_xor_sync(0xffffffffu, x.d, o));
+    return x;
+  };
+  const dual gx = sum(sk.g.x), gy = sum(sk.g.y), gz = sum(sk.g.z), et = sum(e);
+  const dual de = sum(dp[kParLJEps]), ds = sum(dp[kParLJSigma]);
+  if (!live || gl != 0) return;
+  O.glj[a] = make_dual4(gx, gy, gz, 0.0);
+  O.e_lj[a] = et;
+  O.dp[(long)a * kNParam + kParLJEps] += de;
+  O.dp[(long)a * kNParam + kParLJSigma] += ds;
 }
 
 __global__ void k_adj_lj_special(const ReboParams* P, const ReboTables* Tb, LJParams LP, BondListT<dual> B,
@@ -180,11 +267,35 @@ __global__ void k_adj_lj_special(const ReboParams* P, const ReboTables* Tb, LJPa
     lj_special_task<true>(X, S, Tk, t, status, tan);
 }
 
+// Sums of an atom's special-task records into its accumulators (in list order)
+// and the tasks' parameter derivatives, kReduceLanes lanes an atom, an element
+// each.
 __global__ void k_adj_lj_reduce(BondListT<dual> B, SpecialTasksT<dual> Tk, ForceOutT<dual> O)
 {
   pdl_enter();
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a < B.n) lj_reduce_atom(B, Tk, O, a);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int a = t / kReduceLanes;
+  if (a >= B.n) return;
+  const int nb = B.nb[a];
+  int t0, t1;
+  spc_range(Tk, a, t0, t1);
+  if (t1 <= t0) return;
+  // g (3), energy, A (3 nb), W (nb) from the record, then the parameters
+  const int nrec = 4 + 4 * nb;
+  for (int e = t % kReduceLanes; e < nrec + kNParam; e += kReduceLanes) {
+    dual* dst;
+    if (e < 3) dst = reinterpret_cast<dual*>(O.glj + a) + e;
+    else if (e == 3) dst = O.e_lj + a;
+    else if (e < 4 + 3 * nb) dst = O.A + (long)a * O.mb * 3 + (e - 4);
+    else if (e < nrec) dst = O.W + (long)a * O.mb + (e - 4 - 3 * nb);
+    else dst = O.dp + (long)a * kNParam + (e - nrec);
+    dual acc = *dst;
+    for (int q = t0; q < t1; q++) {
+      const long ro = Tk.trec[q];
+      if (ro >= 0) acc += e < nrec ? Tk.rec[ro + e] : Tk.dp[(long)q * kNParam + (e - nrec)];
+    }
+    *dst = acc;
+  }
 }
 
 __global__ void k_adj_gather(BondListT<dual> B, ForceOutT<dual> O, int with_lj, SpecialTasksT<dual> Tk, dual4* g)
@@ -282,7 +393,7 @@ void adj_free(mdg_ctx* c)
   void* ptrs[] = {w->brv, w->bu, w->bd, w->nco, w->A, w->W, w->er, w->et, w->el, w->dp, w->gown, w->glj, w->g,
                   w->cw, w->trec, w->tmidc, w->tdp, w->tmid, w->tan, w->lx, w->lv, w->la, w->theta, w->dpar,
                   w->cp_pos, w->cp_vel, w->cp_acc, w->cp_img, w->seg_pos, w->fin_pos, w->fin_vel, w->fin_acc,
-                  w->fin_img};
+                  w->fin_img, w->brec};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete w;
@@ -312,7 +423,8 @@ int adj_ensure(mdg_ctx* c)
   const bool lj = c->prm.potentials & MDG_POT_AIREBO_LJ;
   const int ccap = lj ? c->cij.cap : 0, tcap = lj ? c->spc.task_cap : 0;
   const long rcap = lj ? c->spc.rec_cap : 0;
-  if (w->n == n && w->mb == mb && w->ccap == ccap && w->tcap == tcap && w->rcap == rcap) return MDG_OK;
+  if (w->n == n && w->mb == mb && w->ccap == ccap && w->tcap == tcap && w->rcap == rcap && w->brcap == c->bt.rec_cap)
+    return MDG_OK;
   bool ok = adj_realloc(w->brv, (size_t)n * mb) && adj_realloc(w->bu, (size_t)n * mb) &&
             adj_realloc(w->bd, (size_t)n * mb) && adj_realloc(w->nco, (size_t)n) &&
             adj_realloc(w->A, (size_t)n * mb * 3) && adj_realloc(w->W, (size_t)n * mb) &&
@@ -326,7 +438,8 @@ int adj_ensure(mdg_ctx* c)
             adj_realloc(w->lx, (size_t)n) && adj_realloc(w->lv, (size_t)n) && adj_realloc(w->la, (size_t)n) &&
             adj_realloc(w->theta, kNParam) && adj_realloc(w->dpar, 2 * kNParam) &&
             adj_realloc(w->fin_pos, (size_t)n) && adj_realloc(w->fin_vel, (size_t)n) &&
-            adj_realloc(w->fin_acc, (size_t)n) && adj_realloc(w->fin_img, (size_t)n);
+            adj_realloc(w->fin_acc, (size_t)n) && adj_realloc(w->fin_img, (size_t)n) &&
+            adj_realloc(w->brec, 2 * (size_t)c->bt.rec_cap);
   if (!ok) return fail(MDG_ERR_CUDA, "cudaMalloc (adjoint buffers)");
   // the glj of a context without the LJ term stays zero; no task holds a
   // middle bond before the first pass
@@ -337,6 +450,7 @@ int adj_ensure(mdg_ctx* c)
   w->ccap = ccap;
   w->tcap = tcap;
   w->rcap = rcap;
+  w->brcap = c->bt.rec_cap;
   w->have_fwd = false;
   w->cp_cap = 0;
   w->seg_cap = 0;
@@ -379,8 +493,9 @@ int adj_dual_pass(mdg_ctx* c, int transpose = 1)
   O.e_lj = w->el;
   O.dp = w->dp;
   O.jt = transpose;
-  LAUNCH(c, "adj_rebo_tors", k_adj_rebo, nblk(n), kThreads, c->d_rp, c->d_tables, DB, c->tp, rebo ? 1 : 0,
-         tors ? 1 : 0, O, c->d_status);
+  LAUNCH(c, "adj_rebo_tors", k_adj_rebo, nblk(n * kAdjLanes, 64), 64, c->d_rp, c->d_tables, DB, c->tp, rebo ? 1 : 0,
+         tors ? 1 : 0, transpose, c->bt.rbase, w->brec, c->d_status);
+  LAUNCH(c, "adj_bond_reduce", k_adj_bond_reduce, nblk(n * kReduceLanes), kThreads, DB, c->bt.rbase, w->brec, O);
   SpecialTasksT<dual> Tk;
   std::memset(&Tk, 0, sizeof(Tk));
   if (lj) {
@@ -390,8 +505,9 @@ int adj_dual_pass(mdg_ctx* c, int transpose = 1)
     DT.ent = c->cij.ent;
     DT.w = w->cw;
     DT.mask = c->cij.mask;
-    LAUNCH(c, "adj_cij", k_adj_cij, nblk(n), kThreads, DB, c->cij, w->cw);
-    LAUNCH(c, "adj_lj_plain", k_adj_lj_plain, nblk(n), kThreads, c->ljp, DT, S, c->nl[1], w->tan, O);
+    LAUNCH(c, "adj_cij", k_adj_cij, nblk(n * kReduceLanes), kThreads, DB, c->cij, w->cw);
+    LAUNCH(c, "adj_lj_plain", k_adj_lj_plain, nblk(n * kLjGroup), kThreads, c->ljp, DT, S, c->nl[1].cap, c->lj_inr,
+           c->lj_inr_cnt, w->tan, O);
     const SpecialTasks& P = c->spc;
     Tk.cap = P.cap;
     Tk.task_cap = P.task_cap;
@@ -408,7 +524,7 @@ int adj_dual_pass(mdg_ctx* c, int transpose = 1)
     Tk.dp = w->tdp;
     LAUNCH(c, "adj_lj_special", k_adj_lj_special, c->special_blocks, kThreads, c->d_rp, c->d_tables, c->ljp, DB, DT,
            S, Tk, w->tan, c->d_status);
-    LAUNCH(c, "adj_lj_reduce", k_adj_lj_reduce, nblk(n), kThreads, DB, Tk, O);
+    LAUNCH(c, "adj_lj_reduce", k_adj_lj_reduce, nblk(n * kReduceLanes), kThreads, DB, Tk, O);
   }
   LAUNCH(c, "adj_gather", k_adj_gather, nblk(n), kThreads, DB, O, lj ? 1 : 0, Tk, w->g);
   return launch_check(c);

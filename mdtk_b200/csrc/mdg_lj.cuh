@@ -759,36 +759,4 @@ MDG_HD void lj_special_pair_task(const LJT<Real, TB>& X, const State& St, Specia
   Tk.midc[t2] = 0.0;
 }
 
-// Sums atom a's special-task records (in list order) into its accumulators
-// (and, on the adjoint path, the tasks' parameter derivatives).
-template <class Wd>
-MDG_HD void lj_reduce_atom(const BondListT<Wd>& B, const SpecialTasksT<Wd>& Tk, ForceOutT<Wd>& O, int a)
-{
-  const int nb = B.nb[a];
-  const auto g0 = O.glj[a];
-  V3T<Wd> g = v3r<Wd>(g0.x, g0.y, g0.z);
-  Wd e = O.e_lj[a];
-  Wd* A = O.A + (long)a * O.mb * 3;
-  Wd* W = O.W + (long)a * O.mb;
-  int t0, t1;
-  spc_range(Tk, a, t0, t1);
-  for (int t = t0; t < t1; t++) {
-    const long ro = Tk.trec[t];
-    if (ro < 0) continue;
-    if (O.dp && Tk.dp)
-      for (int k = 0; k < kNParam; k++) O.dp[(long)a * kNParam + k] += Tk.dp[(long)t * kNParam + k];
-    const Wd* rec = Tk.rec + ro;
-    g += v3r<Wd>(rec[0], rec[1], rec[2]);
-    e += rec[3];
-    for (int s = 0; s < nb; s++) {
-      A[3 * s] += rec[4 + 3 * s];
-      A[3 * s + 1] += rec[4 + 3 * s + 1];
-      A[3 * s + 2] += rec[4 + 3 * s + 2];
-      W[s] += rec[4 + 3 * nb + s];
-    }
-  }
-  O.glj[a] = make_q4(g.x, g.y, g.z, Wd(0.0));
-  O.e_lj[a] = e;
-}
-
 }  // namespace mdg

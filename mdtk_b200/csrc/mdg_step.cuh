@@ -296,26 +296,18 @@ struct ForceOutT {
 typedef ForceOutT<double> ForceOut;
 
 // REBO (+ torsion) for every bond of atom a, evaluated as the reference's
-// bond (min, max) and routed through a Sink for atom a.  ADJ: the adjoint
-// path (duals; parameter derivatives into O.dp).
-template <bool ADJ = false, class Real, class TB>
+// bond (min, max) and routed through a Sink for atom a.
+template <class Real, class TB>
 MDG_HD void rebo_atom(const ReboT<Real, TB>& R, const TorsParams& TP, int do_rebo, int do_tors,
                       ForceOutT<typename Wide<Real>::T>& O, int a)
 {
   typedef typename Wide<Real>::T Wd;
   const auto& B = R.B;
-  SinkT<Real, ADJ> sink;
+  SinkT<Real> sink;
   sink.a = a;
   sink.g = v3r<Wd>(0.0, 0.0, 0.0);
   sink.A = O.A + (long)a * O.mb * 3;
   sink.W = O.W + (long)a * O.mb;
-  sink.dp = nullptr;
-  sink.jt = 1;
-  if constexpr (ADJ) {
-    sink.jt = O.jt;
-    sink.dp = O.dp + (long)a * kNParam;
-    for (int k = 0; k < kNParam; k++) sink.dp[k] = 0.0;
-  }
   for (int s = 0; s < O.mb * 3; s++) sink.A[s] = 0.0;
   for (int s = 0; s < O.mb; s++) sink.W[s] = 0.0;
   Wd er = 0.0, et = 0.0;
