@@ -261,7 +261,7 @@ __global__ void k_adj_lj_special(const ReboParams* P, const ReboTables* Tb, LJPa
 {
   pdl_enter();
   const int total = spc_total(Tk);
-  ReboT<dual, ReboTables> R{*P, *Tb, B, status};
+  ReboT<dual, ReboTables, false> R{*P, *Tb, B, status};
   LJT<dual, ReboTables> X{LP, R, T};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
     lj_special_task<true>(X, S, Tk, t, status, tan);

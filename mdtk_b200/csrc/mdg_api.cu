@@ -438,9 +438,9 @@ __device__ void rebo_end_task(const ReboT<Real, TB>& R, int do_rebo, double* rec
   sink.pair_on = true;
   sink.glo = v3(0, 0, 0);
   sink.ghi = v3(0, 0, 0);
-  sink.A = rec + 5;
-  sink.W = rec + 5 + 3 * nbm;
-  for (int t = 0; t < 4 * nbm; t++) sink.A[t] = 0.0;  // A and W are contiguous
+  LocalRec L;
+  sink.A = L.open(rec + 5, nbm);  // A and W are contiguous
+  sink.W = sink.A + 3 * nbm;
   const PairGT<Real> p = pair_from_slot<Real>(B, lo * B.mb + s);
   double er = 0.0;
   if (do_rebo) {
@@ -461,6 +461,7 @@ __device__ void rebo_end_task(const ReboT<Real, TB>& R, int do_rebo, double* rec
   const double ox = __shfl_xor_sync(pm, e ? sink.glo.x : sink.ghi.x, 1);
   const double oy = __shfl_xor_sync(pm, e ? sink.glo.y : sink.ghi.y, 1);
   const double oz = __shfl_xor_sync(pm, e ? sink.glo.z : sink.ghi.z, 1);
+  L.close(rec + 5, nbm);
   const V3 g = e ? sink.ghi : sink.glo;
   rec[0] = g.x + ox;
   rec[1] = g.y + oy;
@@ -482,14 +483,15 @@ __device__ void rebo_tors_task(const ReboT<Real, TB>& R, const TorsParams& TP, d
   sink.b = hi;
   sink.ga = v3(0, 0, 0);
   sink.gb = v3(0, 0, 0);
-  sink.Aa = rlo + 5;
-  sink.Wa = rlo + 5 + 3 * na;
-  sink.Ab = rhi + 5;
-  sink.Wb = rhi + 5 + 3 * nb;
-  for (int t = 0; t < 4 * na; t++) sink.Aa[t] = 0.0;
-  for (int t = 0; t < 4 * nb; t++) sink.Ab[t] = 0.0;
+  LocalRec La, Lb;
+  sink.Aa = La.open(rlo + 5, na);
+  sink.Wa = sink.Aa + 3 * na;
+  sink.Ab = Lb.open(rhi + 5, nb);
+  sink.Wb = sink.Ab + 3 * nb;
   const PairGT<Real> p = pair_from_slot<Real>(B, lo * B.mb + s);
   const double et = dbl(etors_bond(R, TP, lo, hi, p, sink));
+  La.close(rlo + 5, na);
+  Lb.close(rhi + 5, nb);
   rlo[0] = sink.ga.x;
   rlo[1] = sink.ga.y;
   rlo[2] = sink.ga.z;
@@ -680,9 +682,9 @@ __device__ void brenner_end_task(const Brenner& R, double* rec, int e, int lo, i
   sink.pair_on = true;
   sink.glo = v3(0, 0, 0);
   sink.ghi = v3(0, 0, 0);
-  sink.A = rec + 5;
-  sink.W = rec + 5 + 3 * nbm;
-  for (int t = 0; t < 4 * nbm; t++) sink.A[t] = 0.0;
+  LocalRec L;
+  sink.A = L.open(rec + 5, nbm);
+  sink.W = sink.A + 3 * nbm;
   const PairG p = pair_from_slot(B, lo * B.mb + s);
   Sink dummy;
   const double vav = R.Vexp(lo, hi, p, true, 0.0, dummy);
@@ -694,6 +696,7 @@ __device__ void brenner_end_task(const Brenner& R, double* rec, int e, int lo, i
   const double ox = __shfl_xor_sync(pm, e ? sink.glo.x : sink.ghi.x, 1);
   const double oy = __shfl_xor_sync(pm, e ? sink.glo.y : sink.ghi.y, 1);
   const double oz = __shfl_xor_sync(pm, e ? sink.glo.z : sink.ghi.z, 1);
+  L.close(rec + 5, nbm);
   const V3 g = e ? sink.ghi : sink.glo;
   rec[0] = g.x + ox;
   rec[1] = g.y + oy;
@@ -1195,7 +1198,7 @@ __global__ void k_lj_special(const ReboParams* P, const TB* Tb, LJParams LP, Bon
 {
   pdl_enter();
   const int total = spc_total(Tk);
-  ReboT<Real, TB> R{*P, *Tb, B, status};
+  ReboT<Real, TB, false> R{*P, *Tb, B, status};
   LJT<Real, TB> X{LP, R, T};
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x)
     lj_special_task(X, S, Tk, t, status);
@@ -1212,7 +1215,7 @@ __global__ void k_lj_special_pair(const ReboParams* P, const TB* Tb, LJParams LP
 {
   pdl_enter();
   const long total = (long)min(Tk.ctr[0], (unsigned long long)Tk.task_cap);
-  ReboT<Real, TB> R{*P, *Tb, B, status};
+  ReboT<Real, TB, false> R{*P, *Tb, B, status};
   LJT<Real, TB> X{LP, R, T};
   const int lane = threadIdx.x & 31;
   const long stride = (long)gridDim.x * blockDim.x;

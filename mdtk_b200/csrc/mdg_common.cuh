@@ -190,6 +190,25 @@ template <> struct IsDual<dual> { static constexpr bool v = true; };
 struct dual4 {
   dual x, y, z, w;
 };
+
+// Loads of data that no thread of the running kernel writes (bonds, parameters,
+// tables).  The evaluation writes its records between such loads; as the
+// compiler cannot know that a record never overlaps them, plain loads are
+// repeated after every record update.
+#if defined(__CUDA_ARCH__)
+template <class T>
+MDG_DEV T ro(const T* p) { return __ldg(p); }
+MDG_DEV double4 ro(const double4* p)
+{
+  const double2 a = __ldg(reinterpret_cast<const double2*>(p)), b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+  return make_double4(a.x, a.y, b.x, b.y);
+}
+MDG_DEV dual ro(const dual* p) { return *p; }
+MDG_DEV dual4 ro(const dual4* p) { return *p; }
+#else
+template <class T>
+inline T ro(const T* p) { return *p; }
+#endif
 template <class W> struct Q4T { typedef double4 T; };
 template <> struct Q4T<dual> { typedef dual4 T; };
 MDG_HD dual4 make_dual4(dual x, dual y, dual z, dual w) { dual4 r; r.x = x; r.y = y; r.z = z; r.w = w; return r; }

@@ -23,8 +23,8 @@
 
 namespace mdg {
 
-template <class Real, class TB, class S>
-MDG_HD Real etors_bond(const ReboT<Real, TB>& R, const TorsParams& TP, int i, int j, const PairGT<Real>& p,
+template <class Real, class TB, bool RO, class S>
+MDG_HD Real etors_bond(const ReboT<Real, TB, RO>& R, const TorsParams& TP, int i, int j, const PairGT<Real>& p,
                         S& sink)
 {
   if (R.type(i) != kC || R.type(j) != kC) return 0.0;
@@ -32,21 +32,21 @@ MDG_HD Real etors_bond(const ReboT<Real, TB>& R, const TorsParams& TP, int i, in
   const V3T<Real> a = p.rv;
   const Real wij = p.f;
   Real E = 0.0;
-  const int nbi = B.nb[i], nbj = B.nb[j];
+  const int nbi = R.ld(&B.nb[i]), nbj = R.ld(&B.nb[j]);
   for (int si = 0; si < nbi; si++) {
     const int qi = i * B.mb + si;
-    const int k = B.bj[qi];
+    const int k = R.ld(&B.bj[qi]);
     if (k == j) continue;
-    const auto rk = B.brv[qi], uk = B.bu[qi];
+    const auto rk = R.ld(&B.brv[qi]), uk = R.ld(&B.bu[qi]);
     const V3T<Real> b = xyz<Real>(rk);  // x_i - x_k
     const Real wki = uk.w;
+    const Real sin_ki = sqrt(norm2(cross(a, -b))) / (p.r * rk.w);
+    if (fabs(sin_ki) < 0.1) continue;
     for (int sj = 0; sj < nbj; sj++) {
       const int qj = j * B.mb + sj;
-      const int l = B.bj[qj];
+      const int l = R.ld(&B.bj[qj]);
       if (l == i || l == k) continue;
-      Real sin_ki = sqrt(norm2(cross(a, -b))) / (p.r * rk.w);
-      if (fabs(sin_ki) < 0.1) continue;
-      const auto rl = B.brv[qj], ul = B.bu[qj];
+      const auto rl = R.ld(&B.brv[qj]), ul = R.ld(&B.bu[qj]);
       const V3T<Real> c = xyz<Real>(rl);  // x_j - x_l
       Real sin_jl = sqrt(norm2(cross(a, c))) / (p.r * rl.w);
       if (fabs(sin_jl) < 0.1) continue;
@@ -89,7 +89,7 @@ MDG_HD Real etors_bond(const ReboT<Real, TB>& R, const TorsParams& TP, int i, in
         }
       }
       // ki.f / ij.f / jl.f seeds (AIREBO_ETors.cxx:80-85)
-      Real dfk = B.bd[qi].x, dfl = B.bd[qj].x;
+      Real dfk = R.ld(&B.bd[qi].x), dfl = R.ld(&B.bd[qj].x);
       if (dfk != 0.0) sink.cbond(i, si, xyz<Real>(uk) * ((wij * wjl * val) * dfk));
       if (p.df != 0.0) sink.pair(i, j, p.u * ((wki * wjl * val) * p.df));
       if (dfl != 0.0) sink.cbond(j, sj, xyz<Real>(ul) * ((wki * wij * val) * dfl));

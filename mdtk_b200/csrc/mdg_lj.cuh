@@ -319,7 +319,7 @@ template <class Real, class TB>
 struct LJT {
   typedef typename Wide<Real>::T Wd;
   const LJParams& P;
-  const ReboT<Real, TB>& R;
+  const ReboT<Real, TB, false>& R;
   const CijTableT<Wd>& T;
 
   // b*_ij: REBO's b_ij average for the pair with r_alter = R1 of REBO

@@ -184,22 +184,36 @@ struct EndSinkT {
   }
 };
 
-template <class Real, class TB>
+// RO: bonds and parameters by read-only loads (ro()), which the compiler keeps
+// over the record updates in between: the bond tasks gain by it (43,680 ethane
+// atoms: 100 -> 73 us), the special LJ pairs, which update little, lose (69 ->
+// 81 us: loads are moved up in front of branches that are rarely taken).
+template <class Real, class TB, bool RO = true>
 struct ReboT {
   typedef typename Wide<Real>::T Wd;
+  // Terms that are exact zeros are skipped, but not in float: the float path's
+  // products and sums are contracted block by block, so leaving a block out
+  // moves its results by a rounding.
+  static constexpr bool kSkip = !std::is_same<Real, f32>::value;
+  template <class T>
+  MDG_HD static T ld(const T* p)
+  {
+    if constexpr (RO) return ro(p);
+    else return *p;
+  }
   const ReboParams& P;
   const TB& T;
   const BondListT<Wd>& B;
   unsigned int* status;
 
-  MDG_HD int type(int i) const { return (int)val(B.nco[i].w); }
-  MDG_HD double R2(int ti, int tj) const { return P.R[ti][tj][1]; }
+  MDG_HD int type(int i) const { return (int)val(ld(&B.nco[i].w)); }
+  MDG_HD double R2(int ti, int tj) const { return ld(&P.R[ti][tj][1]); }
 
   // ---- coordination numbers (REBO::Nt/NH/NC, REBO.cxx:423-502) ----
   // which: 0 = all neighbours (Nt), 1 = H only (NH), 2 = C only (NC).
   MDG_HD Real Nval(int c, int o, const PairGT<Real>& p, int which) const
   {
-    const auto n = B.nco[c];
+    const auto n = ld(&B.nco[c]);
     Real N = which == 0 ? n.x : (which == 1 ? n.z : n.y);
     int to = type(o);
     bool sub = (which == 0) || (which == 1 && to == kH) || (which == 2 && to == kC);
@@ -215,19 +229,19 @@ struct ReboT {
   MDG_HD void dfthem(int c, int o, Real V, int which, S& sink) const
   {
     if (V == 0.0) return;
-    const int nb = B.nb[c];
+    const int nb = ld(&B.nb[c]);
     for (int s = 0; s < nb; s++) {
       const int q = c * B.mb + s;
-      const int k = B.bj[q];
+      const int k = ld(&B.bj[q]);
       if (k == o) continue;
       if (which) {
         int tk = type(k);
         if (which == 1 && tk != kH) continue;
         if (which == 2 && tk != kC) continue;
       }
-      Real df = B.bd[q].x;
+      Real df = ld(&B.bd[q].x);
       if (df != 0.0) {
-        const auto u = B.bu[q];
+        const auto u = ld(&B.bu[q]);
         sink.cbond(c, s, xyz<Real>(u) * (V * df));
       }
     }
@@ -250,10 +264,20 @@ struct ReboT {
     if (cost > 1.0) cost = 1.0;
     Real Vc = 0.0, val;
     if (type(c) == kC) {
-      Real g1 = g_eval(T.G[0], cost, 0);
-      Real g2 = g_eval(T.G[1], cost, 0);
+      // with S' = 0 (three neighbours or more) G_C2 alone stays; its terms with
+      // S' are exact zeros
+      const bool both = !kSkip || Sp != 0.0 || SpDer != 0.0;
+      Real g1, g2;
+      if (!kSkip) {
+        g1 = g_eval(T.G[0], cost, 0);
+        g2 = g_eval(T.G[1], cost, 0);
+      } else {
+        g1 = g2 = g_eval(T.G[1], cost, 0);
+        if (both) g1 = g_eval(T.G[0], cost, 0);
+      }
       if (V != 0.0) {
-        Real g1d = g_eval(T.G[0], cost, 1);
+        Real g1d = 0.0;
+        if (both) g1d = g_eval(T.G[0], cost, 1);
         Real g2d = g_eval(T.G[1], cost, 1);
         if (g2d != 0.0 || g1d != 0.0) Vc = g2d * V + g1d * Sp * V + (-g2d * Sp * V);
         if ((g2 != 0.0 || g1 != 0.0) && SpDer != 0.0) dfthem(c, o, g1 * SpDer * V + (-g2 * SpDer * V), 0, sink);
@@ -283,7 +307,7 @@ struct ReboT {
     if (type(c) != kH) return 1.0;
     int tc = type(c), to = type(o), tk = type(k);
     Real rij = p.alter ? p.ralt : p.r;
-    return exp(4.0 * ((P.rho[tc][tk] - bk_r) - (P.rho[tc][to] - rij)));
+    return exp(4.0 * ((ld(&P.rho[tc][tk]) - bk_r) - (ld(&P.rho[tc][to]) - rij)));
   }
 
   // D_co = 1 + sum_k G f_ck lambda + P_co (REBO::D, REBO.cxx:235-265), value.
@@ -292,14 +316,14 @@ struct ReboT {
     SinkT<Real> dummy;
     Real Dij = 1.0;
     Real Nco = Nval(c, o, p, 0);
-    const Real Sp = type(c) == kC ? Sprime(Nco, P.Ntot[0], P.Ntot[1]) : Real(0.0);
-    const int nb = B.nb[c];
+    const Real Sp = type(c) == kC ? Sprime(Nco, ld(&P.Ntot[0]), ld(&P.Ntot[1])) : Real(0.0);
+    const int nb = ld(&B.nb[c]);
     for (int s = 0; s < nb; s++) {
       const int q = c * B.mb + s;
-      const int k = B.bj[q];
+      const int k = ld(&B.bj[q]);
       if (k == o) continue;
-      const auto rv = B.brv[q];
-      const auto u = B.bu[q];
+      const auto rv = ld(&B.brv[q]);
+      const auto u = ld(&B.bu[q]);
       Real ex = expterm(c, o, p, k, rv.w);
       if (ex != 0.0) {
         Real gv = G(c, o, p, s, xyz<Real>(rv), rv.w, xyz<Real>(u), Sp, Real(0.0), 0.0, dummy);
@@ -316,23 +340,27 @@ struct ReboT {
   {
     Real Nco = Nval(c, o, p, 0);
     const bool ccen = type(c) == kC;
-    const Real Sp = ccen ? Sprime(Nco, P.Ntot[0], P.Ntot[1]) : Real(0.0);
-    const Real SpDer = ccen ? dSprime(Nco, P.Ntot[0], P.Ntot[1]) : Real(0.0);
-    const int nb = B.nb[c];
+    const Real Sp = ccen ? Sprime(Nco, ld(&P.Ntot[0]), ld(&P.Ntot[1])) : Real(0.0);
+    const int nb = ld(&B.nb[c]);
+    // without a bond in its switching region nothing follows N_co
+    bool soft = !kSkip;
+    if (kSkip)
+      for (int s = 0; s < nb; s++) soft |= Real(ld(&B.bd[c * B.mb + s].x)) != 0.0;
+    const Real SpDer = ccen && soft ? dSprime(Nco, ld(&P.Ntot[0]), ld(&P.Ntot[1])) : Real(0.0);
     const bool hcen = type(c) == kH;
     for (int s = 0; s < nb; s++) {
       const int q = c * B.mb + s;
-      const int k = B.bj[q];
+      const int k = ld(&B.bj[q]);
       if (k == o) continue;
-      const auto rv = B.brv[q];
-      const auto u = B.bu[q];
+      const auto rv = ld(&B.brv[q]);
+      const auto u = ld(&B.bu[q]);
       V3T<Real> brv = xyz<Real>(rv), bu3 = xyz<Real>(u);
       Real ex = expterm(c, o, p, k, rv.w);
       if (ex == 0.0) continue;
       // one evaluation: the value G returns does not depend on the seed
       Real fv = u.w;
       Real gv = G(c, o, p, s, brv, rv.w, bu3, Sp, SpDer, fv * ex * V, sink);
-      Real df = B.bd[q].x;
+      Real df = ld(&B.bd[q].x);
       if (df != 0.0) sink.cbond(c, s, bu3 * ((gv * ex * V) * df));
       if (hcen) {
         Real Vx = gv * fv * V;
@@ -343,7 +371,7 @@ struct ReboT {
         }
       }
     }
-    P_term(c, o, p, V, sink);
+    if (soft) P_term(c, o, p, V, sink);
   }
 
   // P_co (REBO::P, REBO.cxx:626-657): bicubic in (N^H, N^C) for a carbon centre.
@@ -382,14 +410,14 @@ struct ReboT {
   MDG_HD Real nconj_sum(int c, int o) const
   {
     Real sum = 0.0;
-    const int nb = B.nb[c];
+    const int nb = ld(&B.nb[c]);
     for (int s = 0; s < nb; s++) {
       const int q = c * B.mb + s;
-      const int k = B.bj[q];
+      const int k = ld(&B.bj[q]);
       if (k == o || type(k) != kC) continue;
-      Real f = B.bu[q].w;
-      Real N = Nk_excl(k, B.brv[q].w, f, c);
-      sum += f * Sprime(N, P.Ntot[0], P.Ntot[1]);
+      Real f = ld(&B.bu[q].w);
+      Real N = Nk_excl(k, ld(&B.brv[q].w), f, c);
+      sum += f * Sprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1]));
     }
     return sum;
   }
@@ -397,7 +425,7 @@ struct ReboT {
   // N_kc = Nt_k - f_kc (the pair k-c seen from k), clamped at 0.
   MDG_HD Real Nk_excl(int k, Real r, Real f, int c) const
   {
-    Real N = B.nco[k].x;
+    Real N = ld(&B.nco[k].x);
     if (r < R2(type(k), type(c))) N -= f;
     if (!(N > -n_neg_tol(N))) *status |= ST_N_NEGATIVE;
     if (N < 0) N = 0;
@@ -407,18 +435,18 @@ struct ReboT {
   template <class S>
   MDG_HD void nconj_sum_grad(int c, int o, Real V, S& sink) const
   {
-    const int nb = B.nb[c];
+    const int nb = ld(&B.nb[c]);
     for (int s = 0; s < nb; s++) {
       const int q = c * B.mb + s;
-      const int k = B.bj[q];
+      const int k = ld(&B.bj[q]);
       if (k == o || type(k) != kC) continue;
-      const auto u = B.bu[q];
+      const auto u = ld(&B.bu[q]);
       Real f = u.w;
-      Real N = Nk_excl(k, B.brv[q].w, f, c);
-      Real Sp = Sprime(N, P.Ntot[0], P.Ntot[1]);
-      Real df = B.bd[q].x;
+      Real N = Nk_excl(k, ld(&B.brv[q].w), f, c);
+      Real Sp = Sprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1]));
+      Real df = ld(&B.bd[q].x);
       if (df != 0.0) sink.cbond(c, s, xyz<Real>(u) * ((Sp * V) * df));
-      Real w = f * dSprime(N, P.Ntot[0], P.Ntot[1]) * V;
+      Real w = f * dSprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1])) * V;
       if (w != 0.0) sink.wt(c, s, w);
     }
   }
@@ -446,28 +474,28 @@ struct ReboT {
   MDG_HD Real dh_sum(int i, int j, const PairGT<Real>& p, Real V, S& sink) const
   {
     Real tsum = 0.0;
-    const int nbi = B.nb[i], nbj = B.nb[j];
+    const int nbi = ld(&B.nb[i]), nbj = ld(&B.nb[j]);
     const V3T<Real> a = p.rv;
     for (int si = 0; si < nbi; si++) {
       const int qi = i * B.mb + si;
-      const int k = B.bj[qi];
+      const int k = ld(&B.bj[qi]);
       if (k == j) continue;
-      const auto rk = B.brv[qi];
+      const auto rk = ld(&B.brv[qi]);
       const V3T<Real> b = xyz<Real>(rk);  // x_i - x_k
       for (int sj = 0; sj < nbj; sj++) {
         const int qj = j * B.mb + sj;
-        const int l = B.bj[qj];
+        const int l = ld(&B.bj[qj]);
         if (l == i) continue;
         if (k == l) continue;
         Real sin_ik = sqrt(norm2(cross(a, -b))) / (p.r * rk.w);
         if (fabs(sin_ik) < 0.1) continue;
-        const auto rl = B.brv[qj];
+        const auto rl = ld(&B.brv[qj]);
         const V3T<Real> cc = xyz<Real>(rl);  // x_j - x_l
         Real sin_jl = sqrt(norm2(cross(a, -cc))) / (p.r * rl.w);
         if (fabs(sin_jl) < 0.1) continue;
         int ti = type(i), tk = type(k), tj = type(j), tl = type(l);
-        Real fik = Sprime(Real(rk.w), P.Rp[ti][tk][0], P.Rp[ti][tk][1]);
-        Real fjl = Sprime(Real(rl.w), P.Rp[tj][tl][0], P.Rp[tj][tl][1]);
+        Real fik = Sprime(Real(rk.w), ld(&P.Rp[ti][tk][0]), ld(&P.Rp[ti][tk][1]));
+        Real fjl = Sprime(Real(rl.w), ld(&P.Rp[tj][tl][0]), ld(&P.Rp[tj][tl][1]));
         // cos of the dihedral (FGeneral::CosDihedral, FGeneral.hpp:197-305)
         V3T<Real> u = cross(-a, b);
         V3T<Real> w = cross(a, cc);
@@ -494,14 +522,14 @@ struct ReboT {
             sink.cbond(j, sj, dc * Vd);
           }
           Real vk = (1.0 - SQR(cdh)) * fjl * V;
-          if (vk != 0.0 && rk.w >= P.Rp[ti][tk][0] && rk.w <= P.Rp[ti][tk][1]) {
-            const auto uk = B.bu[qi];
-            sink.cbond(i, si, xyz<Real>(uk) * (dSprime(Real(rk.w), P.Rp[ti][tk][0], P.Rp[ti][tk][1]) * vk));
+          if (vk != 0.0 && rk.w >= ld(&P.Rp[ti][tk][0]) && rk.w <= ld(&P.Rp[ti][tk][1])) {
+            const auto uk = ld(&B.bu[qi]);
+            sink.cbond(i, si, xyz<Real>(uk) * (dSprime(Real(rk.w), ld(&P.Rp[ti][tk][0]), ld(&P.Rp[ti][tk][1])) * vk));
           }
           Real vl = (1.0 - SQR(cdh)) * fik * V;
-          if (vl != 0.0 && rl.w >= P.Rp[tj][tl][0] && rl.w <= P.Rp[tj][tl][1]) {
-            const auto ul = B.bu[qj];
-            sink.cbond(j, sj, xyz<Real>(ul) * (dSprime(Real(rl.w), P.Rp[tj][tl][0], P.Rp[tj][tl][1]) * vl));
+          if (vl != 0.0 && rl.w >= ld(&P.Rp[tj][tl][0]) && rl.w <= ld(&P.Rp[tj][tl][1])) {
+            const auto ul = ld(&B.bu[qj]);
+            sink.cbond(j, sj, xyz<Real>(ul) * (dSprime(Real(rl.w), ld(&P.Rp[tj][tl][0]), ld(&P.Rp[tj][tl][1])) * vl));
           }
         }
         tsum += (1.0 - SQR(cdh)) * fik * fjl;
@@ -582,7 +610,7 @@ struct ReboT {
     if (f == 0.0) return 0.0;
     int ti = type(i), tj = type(j);
     const Wd r = p.rd;
-    const double Q = P.Q[ti][tj], A = P.A[ti][tj], al = P.alpha[ti][tj];
+    const double Q = ld(&P.Q[ti][tj]), A = ld(&P.A[ti][tj]), al = ld(&P.alpha[ti][tj]);
     const Wd t1 = A * exp(-al * r);
     const Wd val = (1 + Q / r) * t1;
     if (V != 0.0) {
@@ -598,11 +626,11 @@ struct ReboT {
   {
     int ti = type(i), tj = type(j);
     const Wd r = p.rd;
-    const Wd t1 = P.B[0][ti][tj] * exp(-P.beta[0][ti][tj] * r);
-    const Wd t2 = P.B[1][ti][tj] * exp(-P.beta[1][ti][tj] * r);
-    const Wd t3 = P.B[2][ti][tj] * exp(-P.beta[2][ti][tj] * r);
+    const Wd t1 = ld(&P.B[0][ti][tj]) * exp(-ld(&P.beta[0][ti][tj]) * r);
+    const Wd t2 = ld(&P.B[1][ti][tj]) * exp(-ld(&P.beta[1][ti][tj]) * r);
+    const Wd t3 = ld(&P.B[2][ti][tj]) * exp(-ld(&P.beta[2][ti][tj]) * r);
     val = t1 + t2 + t3;
-    der = (-P.beta[0][ti][tj]) * t1 + (-P.beta[1][ti][tj]) * t2 + (-P.beta[2][ti][tj]) * t3;
+    der = (-ld(&P.beta[0][ti][tj])) * t1 + (-ld(&P.beta[1][ti][tj])) * t2 + (-ld(&P.beta[2][ti][tj])) * t3;
   }
   template <class S>
   MDG_HD Real VA_from(int i, int j, const PairGT<Real>& p, Wd val, Wd der, Real V, S& sink) const
@@ -644,8 +672,8 @@ struct ReboT {
       // A, alpha, B1, beta1)
       if (type(i) == kC && type(j) == kC && p.f != 0.0) {
         const Wd r = p.rd, f = dbl(p.f);
-        const double Q = P.Q[kC][kC], A = P.A[kC][kC], al = P.alpha[kC][kC];
-        const double B1 = P.B[0][kC][kC], be1 = P.beta[0][kC][kC];
+        const double Q = ld(&P.Q[kC][kC]), A = ld(&P.A[kC][kC]), al = ld(&P.alpha[kC][kC]);
+        const double B1 = ld(&P.B[0][kC][kC]), be1 = ld(&P.beta[0][kC][kC]);
         const Wd eR = f * (1 + Q / r) * exp(-al * r);  // d(f V_R)/dA
         const Wd e1 = f * exp(-be1 * r);                 // -d(f V_A)/dB1
         sink.par(i, kParReboA, eR);
@@ -664,7 +692,7 @@ template <class Real = double>
 MDG_HD PairGT<Real> pair_from_slot(const BondListT<typename Wide<Real>::T>& B, int q)
 {
   PairGT<Real> p;
-  const auto rv = B.brv[q], u = B.bu[q], d = B.bd[q];
+  const auto rv = ro(&B.brv[q]), u = ro(&B.bu[q]), d = ro(&B.bd[q]);
   p.rv = xyz<Real>(rv);
   p.u = xyz<Real>(u);
   p.r = rv.w;

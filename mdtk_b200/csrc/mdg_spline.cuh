@@ -58,13 +58,16 @@ struct ReboTables {
 
 // 1-D quintic piece: sum_t coef[t] * x^(t - d), d = 0 for the value poly and
 // 1 for the derivative poly (whose term 0 is always zero).
+// A term whose coefficient is 0 adds 0 instead of being skipped: the same sum,
+// without a branch between the loads of consecutive terms.
 MDG_HD double poly1(const double* c, double x, int deriv)
 {
-  double val = 0.0;
+  double val = 0.0, p = 1.0;
+#pragma unroll
   for (int t = 0; t < 6; t++) {
-    double ct = c[t];
-    if (ct == 0.0) continue;
-    val = add_rn(val, mul_rn(ct, ipow(x, t - deriv)));
+    if (t < deriv) continue;
+    val = add_rn(val, mul_rn(ro(c + t), p));
+    p = mul_rn(p, x);
   }
   return val;
 }

@@ -355,6 +355,28 @@ struct BondTasks {
 
 MDG_HD int bond_rec_size(int nb) { return 5 + 4 * nb; }
 
+// The A and W part of a record while its task runs: in the thread's own memory
+// (kept in L1; a record in global memory would write every update through to
+// L2), copied out once at the end.  An atom with more than kLocalBonds bonds
+// accumulates in its record.  The bond tasks of 43,680 ethane atoms: 84 us
+// with the records updated in place, 73 so; the special LJ pairs, which update
+// theirs a few times at most, are better off without.
+constexpr int kLocalBonds = 16;
+struct LocalRec {
+  double acc[4 * kLocalBonds];
+  MDG_HD double* open(double* rec, int nb)
+  {
+    double* A = nb <= kLocalBonds ? acc : rec;
+    for (int t = 0; t < 4 * nb; t++) A[t] = 0.0;
+    return A;
+  }
+  MDG_HD void close(double* rec, int nb) const
+  {
+    if (nb <= kLocalBonds)
+      for (int t = 0; t < 4 * nb; t++) rec[t] = acc[t];
+  }
+};
+
 template <class Real, class TB>
 MDG_HD void rebo_task(const ReboT<Real, TB>& R, const TorsParams& TP, int do_rebo, int do_tors, double* rec, int a,
                       int s)
@@ -364,9 +386,9 @@ MDG_HD void rebo_task(const ReboT<Real, TB>& R, const TorsParams& TP, int do_reb
   SinkT<Real> sink;
   sink.a = a;
   sink.g = v3(0, 0, 0);
-  sink.A = rec + 5;
-  sink.W = rec + 5 + 3 * nb;
-  for (int t = 0; t < 4 * nb; t++) sink.A[t] = 0.0;  // A and W are contiguous
+  LocalRec L;
+  sink.A = L.open(rec + 5, nb);  // A and W are contiguous
+  sink.W = sink.A + 3 * nb;
   const int q = a * B.mb + s;
   const int b = B.bj[q];
   PairGT<Real> p = pair_from_slot<Real>(B, q);
@@ -381,6 +403,7 @@ MDG_HD void rebo_task(const ReboT<Real, TB>& R, const TorsParams& TP, int do_reb
     const Real E = etors_bond(R, TP, lo, hi, p, sink);
     if (a == lo) et = dbl(E);
   }
+  L.close(rec + 5, nb);
   rec[0] = sink.g.x;
   rec[1] = sink.g.y;
   rec[2] = sink.g.z;
@@ -401,16 +424,17 @@ MDG_HD void rebo_pair_task(const ReboT<Real, TB>& R, const TorsParams& TP, int d
   sink.b = hi;
   sink.ga = v3(0, 0, 0);
   sink.gb = v3(0, 0, 0);
-  sink.Aa = rlo + 5;
-  sink.Wa = rlo + 5 + 3 * na;
-  sink.Ab = rhi + 5;
-  sink.Wb = rhi + 5 + 3 * nb;
-  for (int t = 0; t < 4 * na; t++) sink.Aa[t] = 0.0;
-  for (int t = 0; t < 4 * nb; t++) sink.Ab[t] = 0.0;
+  LocalRec La, Lb;
+  sink.Aa = La.open(rlo + 5, na);
+  sink.Wa = sink.Aa + 3 * na;
+  sink.Ab = Lb.open(rhi + 5, nb);
+  sink.Wb = sink.Ab + 3 * nb;
   const PairGT<Real> p = pair_from_slot<Real>(B, lo * B.mb + s);
   double er = 0.0, et = 0.0;
   if (do_rebo) er = dbl(R.bond(lo, hi, p, sink));
   if (do_tors) et = dbl(etors_bond(R, TP, lo, hi, p, sink));
+  La.close(rlo + 5, na);
+  Lb.close(rhi + 5, nb);
   rlo[0] = sink.ga.x;
   rlo[1] = sink.ga.y;
   rlo[2] = sink.ga.z;
