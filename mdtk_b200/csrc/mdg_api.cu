@@ -1081,6 +1081,7 @@ __device__ __forceinline__ void lj_pairs_block(const LJParams& P, const CijTable
   const double4 pa = S.pos[a];
   const V3 xa = v3(pa.x, pa.y, pa.z);
   const int ta = (int)pa.w;
+  const Box box = box_of(S, a);
   const int nc = live ? close_cnt[a] : 0;
   const int nf = live ? far_cnt[a] : 0;
   const unsigned long long amask = T.mask[a];
@@ -1125,7 +1126,10 @@ __device__ __forceinline__ void lj_pairs_block(const LJParams& P, const CijTable
     int b = -1, kind = 0;
     if (s < nf) {
       b = row[s];
-      kind = lj_plain_pair<Real>(P, T, S, a, b, xa, ta, amask, sk, e, nullptr, true);
+      if constexpr (std::is_same<Real, double>::value)
+        kind = lj_far_pair(P, T, S, a, b, xa, ta, box, amask, sk.g, e);
+      else
+        kind = lj_plain_pair<Real>(P, T, S, a, b, xa, ta, amask, sk, e, nullptr, true);
     }
     note(kind == 2, b);
   }

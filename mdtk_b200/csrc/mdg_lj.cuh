@@ -595,6 +595,39 @@ MDG_HD LJClass lj_class(const LJParams& P, const CijTableT<W>& T, const State& S
   return c;
 }
 
+// A far pair (outside the S(t_r) window, within the cutoff) seen from atom a in
+// double: its lj_kind; a plain pair adds its gradient on a to g and, at the
+// lower end, its energy to e.  VLJ = 4 eps [(s/r)^12 - (s/r)^6] and (dV/dr)/r
+// are polynomials in 1/r^2, so only the pairs inside the cutoff's cosine window
+// take a root: half of the instructions of the general form (lj_plain_pair),
+// which the float and adjoint paths keep.
+MDG_HD int lj_far_pair(const LJParams& P, const CijTableT<double>& T, const State& St, int a, int b, V3 xa, int ta,
+                       const Box& box, unsigned long long amask, V3& g, double& e)
+{
+  const double4 pb = St.pos[b];
+  const int tb = (int)pb.w;
+  const V3 rv = depos(box, xa, v3(pb.x, pb.y, pb.z));  // (depos is antisymmetric: no order of the ends needed)
+  const double d2 = norm2(rv);
+  const double w = lj_w_own(T, a, b, amask);
+  const int kind = lj_kind(w, false);
+  if (kind != 1) return kind;
+  const double R1 = P.R[ta][tb][0], R2 = P.R[ta][tb][1];
+  const double ir2 = 1.0 / d2, sigma = P.sigma[ta][tb], e4 = 4.0 * P.eps[ta][tb];
+  const double s2 = sigma * sigma * ir2, s6 = s2 * s2 * s2;
+  double v = e4 * (s6 * s6 - s6), q = e4 * (6.0 * s6 - 12.0 * (s6 * s6)) * ir2;
+  if (d2 >= R1 * R1) {
+    const double r = sqrt(d2), iw = 1.0 / (R2 - R1);
+    double sn, cs;
+    sincospi((r - R1) * iw, &sn, &cs);
+    const double f = 0.5 + 0.5 * cs;
+    q = f * q - v * (0.5 * kPi * iw) * sn / r;
+    v *= f;
+  }
+  g += rv * q;
+  if (a < b) e += v;
+  return 1;
+}
+
 // One LJ pair seen from atom a: returns its lj_class kind; for plain pairs
 // adds the own gradient and, at the lower end, the energy.  known_far: the
 // pair is known to lie outside the S(t_r) window (the in-range filter's far
