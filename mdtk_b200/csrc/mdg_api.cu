@@ -769,9 +769,10 @@ constexpr int kCijScratch = 4 * kCijCand;    // ints of a group's scratch row: t
 constexpr int kCijNone = 0x7fffffff;         // no target
 
 // Also zeroes the special-pair counters that the special-pair finder after it
-// hands ranges out of.
+// hands ranges out of, and the atoms' middle-bond flags.
 __global__ void __launch_bounds__(kCijThreads) k_cij(BondList B, CijTable T, int* scratch,
-                                                     unsigned long long* spc_ctr, unsigned int* status)
+                                                     unsigned long long* spc_ctr, unsigned char* mflag,
+                                                     unsigned int* status)
 {
   pdl_enter();
   const int tid = threadIdx.x, gl = tid % kCijGroup, lane = tid & 31, gbase = lane - gl;
@@ -907,6 +908,7 @@ __global__ void __launch_bounds__(kCijThreads) k_cij(BondList B, CijTable T, int
       mhi |= __shfl_xor_sync(0xffffffffu, mhi, o);
     }
     if (live && gl == 0) {
+      mflag[a] = 0;
       if (wide) {
         cij_build_atom<kCijLocal>(B, T, a, status);
       } else {
@@ -1264,6 +1266,9 @@ __device__ V3 gather_lanes(const BondList& B, const ForceOut& O, const SpecialTa
     }
   }
   const int nb = B.nb[a];
+  // middle bonds touch few atoms (none of a molecular system): the tasks of
+  // two shells of neighbours are searched only for those
+  const bool mid = with_lj && X.mflag[a];
   for (int s = l; s < nb; s += kGatherLanes) {
     const int q = a * B.mb + s;
     const int k = B.bj[q];
@@ -1292,7 +1297,7 @@ __device__ V3 gather_lanes(const BondList& B, const ForceOut& O, const SpecialTa
       const double4 u = B.bu[q];
       g += v3(u.x, u.y, u.z) * (df * (wa + wm));
     }
-    if (with_lj) {
+    if (mid) {
       // middle-bond terms of the LJ special pairs (mid_gather_atom)
       int t0, t1;
       spc_range(X, k, t0, t1);
@@ -1943,7 +1948,7 @@ void free_system(mdg_ctx* c)
     c->has_list[l] = false;
   }
   void* lq[] = {c->cij.cnt, c->cij.ent, c->cij.w, c->cij.mask, c->spc.cnt, c->spc.part, c->spc.off,
-                c->spc.flat, c->spc.trec, c->spc.rec, c->spc.mid, c->spc.midc, c->spc.work,
+                c->spc.flat, c->spc.trec, c->spc.rec, c->spc.mid, c->spc.midc, c->spc.mflag, c->spc.work,
                 c->spc.ctr, c->lj_inr, c->lj_inr_cnt, c->ljt.cnt, c->ljt.list, c->ljt.pos0,
                 c->cij_scratch};
   c->cij_scratch = nullptr;
@@ -2293,7 +2298,7 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
     LAUNCH(c, "brenner", k_brenner, nblk(c->n), kThreads, c->d_bp, c->d_btables, B, c->fo, c->d_status);
   if (lj) {
     LAUNCH(c, "cij_table", k_cij, std::min(nblk(c->n, kCijAtoms), c->cij_blocks), kCijThreads, B, c->cij,
-           c->cij_scratch, c->spc.ctr, c->d_status);
+           c->cij_scratch, c->spc.ctr, c->spc.mflag, c->d_status);
     if (ovl) CK(cudaStreamWaitEvent(c->stream, c->ev_join2, 0));
     const int pairs = (c->bt.ctr && c->bt.pairs) ? 1 : 0;
     const int lgrid = nblk(c->n * kLjGroup, kLjThreads);
@@ -2795,13 +2800,14 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     X.trec = dalloc<long>(X.task_cap);
     X.rec = dalloc<double>(X.rec_cap);
     X.mid = dalloc<int4>(X.task_cap);
+    X.mflag = dalloc<unsigned char>(n);
     X.midc = dalloc<double>(X.task_cap);
     X.work = dalloc<int>(X.task_cap);
     X.ctr = dalloc<unsigned long long>(3 * kCtrStride);
     if (!X.work || !X.ctr) return fail(MDG_ERR_CUDA, "cudaMalloc (LJ work list)");
     CK(cudaMemset(X.ctr, 0, 3 * kCtrStride * sizeof(unsigned long long)));
     if (!c->cij.cnt || !c->cij.ent || !c->cij.w || !c->cij.mask || !X.cnt || !X.part || !X.off || !X.flat ||
-        !X.trec || !X.rec || !X.mid || !X.midc)
+        !X.trec || !X.rec || !X.mid || !X.midc || !X.mflag)
       return fail(MDG_ERR_CUDA, "cudaMalloc (LJ)");
     CK(cudaMemset(X.cnt, 0, n * sizeof(int)));
     CK(cudaMemset(X.off, 0, n * sizeof(int)));

@@ -468,6 +468,7 @@ struct SpecialTasksT {
   W* dp;            // [task_cap * kNParam] energy derivatives by parameter (adjoint path only)
   // one evaluation per pair (the lower-index end's task writes both records):
   int* work;        // [task_cap] tasks whose owner is the lower index (-1: beyond task_cap)
+  unsigned char* mflag;     // [n] the atom is an end of a middle bond of some task (FP64 and mixed paths)
   unsigned long long* ctr;  // work items, tasks, record doubles handed out this evaluation, at
                             // ctr[0], ctr[kCtrStride], ctr[2 kCtrStride] (one 128-byte line each)
 };
@@ -737,6 +738,7 @@ MDG_HD void lj_special_task(const LJT<Real, TB>& X, const State& St, SpecialTask
   rec[3] = (a == lo) ? dbl(E) : Wd(0.0);
   Tk.mid[t] = make_int4(mo.k, mo.sm, mo.m, mo.valid);
   Tk.midc[t] = mo.valid ? mo.c : Wd(0.0);
+  if (mo.valid && Tk.mflag) Tk.mflag[mo.k] = Tk.mflag[mo.m] = 1;
 }
 
 // One special pair (a < b) from task t of a and task t2 of b, written into
@@ -788,6 +790,7 @@ MDG_HD void lj_special_pair_task(const LJT<Real, TB>& X, const State& St, Specia
   rb[3] = 0.0;
   Tk.mid[t] = make_int4(mo.k, mo.sm, mo.m, mo.valid);
   Tk.midc[t] = mo.valid ? mo.c : 0.0;
+  if (mo.valid) Tk.mflag[mo.k] = Tk.mflag[mo.m] = 1;
   Tk.mid[t2] = make_int4(0, 0, 0, 0);
   Tk.midc[t2] = 0.0;
 }
