@@ -339,18 +339,26 @@ MDG_HD void cutoff(Real r, double R1, double R2, Real& f, Real& df)
 }
 
 // Sprime / dSprime (REBO.cxx:67-106): 1 below min, 0 above max, cosine between.
+// At the ends themselves Sprime's cosine gives exactly 1 and 0, so they take
+// the constants too: a carbon with three other neighbours sits on one.
+// (dSprime's sine of pi is 1e-16, not 0; it is a coefficient of other bonds'
+// df, all of which are 0 at a whole coordination.)
 template <class Real>
 MDG_HD Real Sprime(Real arg, double amin, double amax)
 {
-  if (arg < amin) return 1.0;
-  if (arg > amax) return 0.0;
+  if (arg <= amin) return 1.0;
+  if (arg >= amax) return 0.0;
   return (1.0 + cos(kPi * (arg - amin) / (amax - amin))) / 2.0;
 }
 template <class Real>
 MDG_HD Real dSprime(Real arg, double amin, double amax)
 {
   if (arg < amin) return 0.0;
-  if (arg > amax) return 0.0;
+  if constexpr (std::is_same<Real, f32>::value) {
+    if (arg > amax) return 0.0;
+  } else {
+    if (arg >= amax) return 0.0;
+  }
   return (-(kPi / (amax - amin)) * sin(kPi * (arg - amin) / (amax - amin))) / 2.0;
 }
 
