@@ -2232,6 +2232,7 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
               c->ljt, c->lj_inr, c->lj_inr_cnt, c->lj_inr_cnt + c->n);
     CK(cudaEventRecord(c->ev_join2, c->side2));
     rc = rebuild_list(c, 0, c->stream);
+    if (!rc) rc = rebuild_list(c, 2, c->stream);
     if (rc) return rc;
   } else {
     rc = rebuild_lists(c, step);
