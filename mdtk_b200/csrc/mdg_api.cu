@@ -197,80 +197,130 @@ __global__ void k_nl_build(State S, Grid g, NList L, const int* need, unsigned i
   if (i < S.n) nl_build_atom(S, g, L, i, status);
 }
 
-__global__ void k_bonds(State S, NList L, ReboParams P, BondBuild B, BondTasks K, unsigned int* status)
+// Lanes per atom of the bond list and the reverse slots: as long as eight times
+// the atoms fit the GPU's resident threads, an atom's list entries are spread
+// over eight lanes; beyond, over two (512,000 diamond atoms: bonds 240 and
+// reverse slots 72 us on eight lanes, 168 and 46 on two; a thread an atom took
+// 164 and 62).
+constexpr int kBondLanes = 8, kBondLanesLarge = 2;
+constexpr int kBondLanesAtoms = 65536;
+
+// The bond list, LANES lanes per atom.  Bound by the latency of the position
+// gathers: a thread an atom walked its ~16 list entries in sequence (1,728
+// diamond atoms: 15 us; so 5).
+template <int LANES>
+__global__ void __launch_bounds__(kThreads) k_bonds(State S, NList L, ReboParams P, BondBuild B, BondTasks K,
+                                                    unsigned int* status)
 {
   pdl_enter();
-  int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a == 0 && K.ctr) K.ctr[0] = K.ctr[1] = K.ctr[2] = 0;
-  if (a < S.n) bonds_atom(S, L, P, B, a, status);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, a = t / LANES;
+  if (t < 3 && K.ctr) K.ctr[t * kTaskCtr] = 0;
+  bonds_atom<LANES>(S, L, P, B, min(a, S.n - 1), a < S.n, status);
 }
 
-// Exclusive offset of this lane's v within a block handed out to the warp by
-// one atomicAdd on *ctr.  All 32 lanes must call it.
-__device__ unsigned long long warp_alloc(unsigned long long v, unsigned long long* ctr)
+// Exclusive offsets of this thread's v[0..2] within ranges handed out to the
+// block by one atomicAdd per counter (ctr[0], ctr[kCtrStride],
+// ctr[2 kCtrStride]).  Every thread of the block (blockDim.x == NT) calls it.
+template <int NT>
+__device__ void block_alloc3(const unsigned long long v[3], unsigned long long* ctr, unsigned long long out[3])
 {
-  const int lane = threadIdx.x & 31;
-  unsigned long long x = v;
-  for (int o = 1; o < 32; o <<= 1) {
-    unsigned long long t = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += t;
+  __shared__ unsigned long long ws[3][NT / 32];
+  __shared__ unsigned long long base[3];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  unsigned long long x[3];
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    x[k] = v[k];
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, x[k], o);
+      if (lane >= o) x[k] += t;
+    }
+    if (lane == 31) ws[k][wid] = x[k];
   }
-  unsigned long long base = 0;
-  if (lane == 31 && x) base = atomicAdd(ctr, x);
-  base = __shfl_sync(0xffffffffu, base, 31);
-  return base + x - v;
+  __syncthreads();
+  if (threadIdx.x < 3) {
+    const int k = threadIdx.x;
+    unsigned long long run = 0;
+    for (int w = 0; w < NT / 32; w++) {
+      const unsigned long long t = ws[k][w];
+      ws[k][w] = run;
+      run += t;
+    }
+    base[k] = run ? atomicAdd(ctr + k * kCtrStride, run) : 0ull;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 3; k++) out[k] = base[k] + ws[k][wid] + x[k] - v[k];
 }
 
 // Reverse slots, then the REBO bond tasks of each atom: record space and the
-// task queue (C-C bonds, which carry the torsion and dihedral terms, first).
-// Positions in the queue and the record pool depend on scheduling; the values
+// task queue (C-C bonds, which carry the torsion and dihedral terms, first),
+// LANES lanes per atom, a bond each (1,728 diamond atoms: 8 us on a thread an
+// atom, 4 so).  Positions in the queue and the
+// record pool depend on scheduling (ranges handed out per block); the values
 // written to each slot's record do not.
-__global__ void k_brev(BondBuild B, BondTasks K, unsigned int* status)
+constexpr int kBrevThreads = 256;
+template <int LANES>
+__global__ void __launch_bounds__(kBrevThreads) k_brev(BondBuild B, BondTasks K, unsigned int* status)
 {
   pdl_enter();
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool ok = a < B.n;
-  int nb = 0, ncc = 0;
-  if (ok) {
-    brev_atom(B, a);
-    if (K.ctr) {
-      nb = B.nb[a];
-      if ((int)B.nco[a].w == kC)
-        for (int s = 0; s < nb; s++) ncc += ((int)B.nco[B.bj[a * B.mb + s]].w == kC);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lane = threadIdx.x & 31, gl = lane % LANES, gbase = lane - gl;
+  const unsigned gmask = ((1u << LANES) - 1u) << gbase, below = ((1u << lane) - 1u) & gmask;
+  const bool ok = t / LANES < B.n;
+  const int a = ok ? t / LANES : B.n - 1;
+  const int nb = ok ? B.nb[a] : 0;
+  const bool carbon = K.ctr && (int)B.nco[a].w == kC;
+  const int most = __reduce_max_sync(0xffffffffu, nb);
+  // queued slots: all (one task per directed slot) or those to higher
+  // partners (one task per bond)
+  int ncc = 0, mcc = 0, mot = 0;
+  for (int base = 0; base < most; base += LANES) {
+    const int s = base + gl;
+    bool cc = false, on = false;
+    if (s < nb) {
+      const int j = B.bj[a * B.mb + s];
+      B.brev[a * B.mb + s] = brev_slot(B, a, j);
+      cc = carbon && (int)B.nco[j].w == kC;
+      on = !(K.pairs && j < a);
     }
+    ncc += __popc(__ballot_sync(0xffffffffu, cc) & gmask);
+    mcc += __popc(__ballot_sync(0xffffffffu, cc && on) & gmask);
+    mot += __popc(__ballot_sync(0xffffffffu, !cc && on) & gmask);
   }
   if (!K.ctr) return;  // uniform over the launch
   // records: one per bond slot, then (split mode with torsion) one per C-C bond
   const int nrec = nb + ((K.pairs == 2 && K.tors) ? ncc : 0);
-  const unsigned long long need = ok ? (unsigned long long)nrec * bond_rec_size(nb) : 0ull;
-  const unsigned long long rb = warp_alloc(need, &K.ctr[2]);
-  // queued slots: all (one task per directed slot) or those to higher
-  // partners (one task per bond)
-  int mcc = 0, mot = 0;
-  if (ok)
-    for (int s = 0; s < nb; s++) {
-      const int j = B.bj[a * B.mb + s];
-      if (K.pairs && j < a) continue;
-      if (ncc && (int)B.nco[j].w == kC) mcc++;
-      else mot++;
+  const unsigned long long need = (unsigned long long)nrec * bond_rec_size(nb);
+  const bool lead = ok && gl == 0;
+  const unsigned long long v[3] = {lead ? (unsigned long long)mcc : 0ull, lead ? (unsigned long long)mot : 0ull,
+                                   lead ? need : 0ull};
+  unsigned long long r[3];
+  block_alloc3<kBrevThreads>(v, K.ctr, r);
+  int f = (int)__shfl_sync(0xffffffffu, r[0], gbase), b = (int)__shfl_sync(0xffffffffu, r[1], gbase);
+  if (lead) {
+    if ((long)(r[2] + need) > K.rec_cap) {
+      K.rbase[a] = -1;
+      atomicOr(status, ST_RECORD_OVERFLOW);
+    } else {
+      K.rbase[a] = (long)r[2];
     }
-  const unsigned long long i0 = warp_alloc(mcc, &K.ctr[0]);
-  const unsigned long long i1 = warp_alloc(mot, &K.ctr[1]);
-  if (!ok) return;
-  if ((long)(rb + need) > K.rec_cap) {
-    K.rbase[a] = -1;
-    atomicOr(status, ST_RECORD_OVERFLOW);
-  } else {
-    K.rbase[a] = (long)rb;
+    K.nrec[a] = nrec;
   }
-  K.nrec[a] = nrec;
-  int f = (int)i0, b = (int)i1;
-  for (int s = 0; s < nb; s++) {
-    const int j = B.bj[a * B.mb + s];
-    if (K.pairs && j < a) continue;
-    const bool cc = ncc && (int)B.nco[j].w == kC;
-    if (cc) K.q[f++] = a * B.mb + s;
-    else K.q[K.cap - 1 - (b++)] = a * B.mb + s;
+  for (int base = 0; base < most; base += LANES) {
+    const int s = base + gl;
+    bool cc = false, on = false;
+    if (s < nb) {
+      const int j = B.bj[a * B.mb + s];
+      cc = carbon && (int)B.nco[j].w == kC;
+      on = !(K.pairs && j < a);
+    }
+    const unsigned mc = __ballot_sync(0xffffffffu, cc && on) & gmask;
+    const unsigned mo = __ballot_sync(0xffffffffu, !cc && on) & gmask;
+    if (cc && on) K.q[f + __popc(mc & below)] = a * B.mb + s;
+    if (!cc && on) K.q[K.cap - 1 - (b + __popc(mo & below))] = a * B.mb + s;
+    f += __popc(mc);
+    b += __popc(mo);
   }
 }
 
@@ -303,7 +353,7 @@ __global__ void __launch_bounds__(128) k_rebo_task(const ReboParams* P, const TB
                                                    int do_rebo, int do_tors, BondTasks K, unsigned int* status)
 {
   pdl_enter();
-  const long n0 = (long)K.ctr[0], nt = n0 + (long)K.ctr[1];
+  const long n0 = (long)K.ctr[0], nt = n0 + (long)K.ctr[kTaskCtr];
   ReboT<Real, TB> R{*P, *T, B, status};
   for (long t = spread_task_index(); t < nt; t += (long)gridDim.x * blockDim.x) {
     const int q = t < n0 ? K.q[t] : K.q[K.cap - 1 - (t - n0)];
@@ -321,7 +371,7 @@ __global__ void __launch_bounds__(128) k_rebo_pair_task(const ReboParams* P, con
                                                         unsigned int* status)
 {
   pdl_enter();
-  const long n0 = (long)K.ctr[0], nt = n0 + (long)K.ctr[1];
+  const long n0 = (long)K.ctr[0], nt = n0 + (long)K.ctr[kTaskCtr];
   ReboT<Real, TB> R{*P, *T, B, status};
   for (long t = spread_task_index(); t < nt; t += (long)gridDim.x * blockDim.x) {
     const int q = t < n0 ? K.q[t] : K.q[K.cap - 1 - (t - n0)];
@@ -521,7 +571,7 @@ __global__ void __launch_bounds__(128) k_rebo_split_task(const ReboParams* P, co
                                                          int do_rebo, int do_tors, BondTasks K, unsigned int* status)
 {
   pdl_enter();
-  const long n0 = (long)K.ctr[0], n1 = (long)K.ctr[1];
+  const long n0 = (long)K.ctr[0], n1 = (long)K.ctr[kTaskCtr];
   const long ntor = do_tors ? n0 : 0;
   const long base1 = (2 * n0 + ntor + 1) & ~1L;
   const long total = base1 + 2 * n1;
@@ -715,7 +765,7 @@ __global__ void __launch_bounds__(128) k_brenner_split_task(const BrennerParams*
                                                             unsigned int* status)
 {
   pdl_enter();
-  const long n0 = (long)K.ctr[0], n1 = (long)K.ctr[1];
+  const long n0 = (long)K.ctr[0], n1 = (long)K.ctr[kTaskCtr];
   const long ntor = do_tors ? n0 : 0;
   const long base1 = (2 * n0 + ntor + 1) & ~1L;
   const long total = base1 + 2 * n1;
@@ -1022,41 +1072,6 @@ __global__ void __launch_bounds__(kThreads) k_lj_filter(LJParams P, State S, NLi
       close_cnt[a] = kc;
     }
   }
-}
-
-// Exclusive offsets of this thread's v[0..2] within ranges handed out to the
-// block by one atomicAdd per counter (ctr[0], ctr[kCtrStride],
-// ctr[2 kCtrStride]).  Every thread of the block (blockDim.x == NT) calls it.
-template <int NT>
-__device__ void block_alloc3(const unsigned long long v[3], unsigned long long* ctr, unsigned long long out[3])
-{
-  __shared__ unsigned long long ws[3][NT / 32];
-  __shared__ unsigned long long base[3];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  unsigned long long x[3];
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    x[k] = v[k];
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xffffffffu, x[k], o);
-      if (lane >= o) x[k] += t;
-    }
-    if (lane == 31) ws[k][wid] = x[k];
-  }
-  __syncthreads();
-  if (threadIdx.x < 3) {
-    const int k = threadIdx.x;
-    unsigned long long run = 0;
-    for (int w = 0; w < NT / 32; w++) {
-      const unsigned long long t = ws[k][w];
-      ws[k][w] = run;
-      run += t;
-    }
-    base[k] = run ? atomicAdd(ctr + k * kCtrStride, run) : 0ull;
-  }
-  __syncthreads();
-#pragma unroll
-  for (int k = 0; k < 3; k++) out[k] = base[k] + ws[k][wid] + x[k] - v[k];
 }
 
 // The LJ pairs of each atom, kLjGroup lanes per atom: the plain pairs of its
@@ -2161,7 +2176,7 @@ int step_start(mdg_ctx* c, const StepDev* step)
   }
   StepDev none;
   std::memset(&none, 0, sizeof(none));
-  LAUNCH(c, step ? "verlet_pos_disp" : "nl_disp", k_step_start, kDispParts, kThreads, S,
+  LAUNCH(c, step ? "verlet_pos_disp" : "nl_disp", k_step_start, std::min(nblk(c->n), kDispParts), kThreads, S,
          step ? *step : none, step ? 1 : 0, c->nl[0], c->nl[1], c->nl[2], c->ljt, mask, c->d_part, c->d_need, c->d_force,
          c->d_disp_done);
   return MDG_OK;
@@ -2241,7 +2256,13 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
       LAUNCH(c, "lj_filter", k_lj_filter, std::min(nblk(c->n * 32), c->warp_blocks), kThreads, c->ljp, S, c->ljt,
              c->lj_inr, c->lj_inr_cnt, c->lj_inr_cnt + c->n);
   }
-  LAUNCH(c, "bonds", k_bonds, nblk(c->n), kThreads, S, c->nl[0], c->rp, c->bb, c->bt, c->d_status);
+  const bool large = c->n > kBondLanesAtoms;
+  if (large)
+    LAUNCH(c, "bonds", k_bonds<kBondLanesLarge>, nblk(c->n * kBondLanesLarge), kThreads, S, c->nl[0], c->rp, c->bb,
+           c->bt, c->d_status);
+  else
+    LAUNCH(c, "bonds", k_bonds<kBondLanes>, nblk(c->n * kBondLanes), kThreads, S, c->nl[0], c->rp, c->bb, c->bt,
+           c->d_status);
   BondList B = c->BL();
   const bool f32p = c->prm.precision == MDG_PREC_FP32_MIXED;
   cudaStream_t rs = c->stream;
@@ -2252,7 +2273,12 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
     CK(cudaStreamWaitEvent(c->side, c->ev_fork, 0));
     rs = c->side;
   }
-  LAUNCH_ON(c, rs, "bonds_rev", k_brev, nblk(c->n), kThreads, c->bb, c->bt, c->d_status);
+  if (large)
+    LAUNCH_ON(c, rs, "bonds_rev", k_brev<kBondLanesLarge>, nblk(c->n * kBondLanesLarge, kBrevThreads), kBrevThreads,
+              c->bb, c->bt, c->d_status);
+  else
+    LAUNCH_ON(c, rs, "bonds_rev", k_brev<kBondLanes>, nblk(c->n * kBondLanes, kBrevThreads), kBrevThreads, c->bb,
+              c->bt, c->d_status);
   if (tasks && (pot & MDG_POT_BRENNER)) {
     LAUNCH(c, "brenner", k_brenner_split_task, c->rebo_task_blocks, kThreads, c->d_bp, c->d_btables, c->d_rp,
            c->d_tables, B, c->tp, tors ? 1 : 0, c->bt, c->d_status);
@@ -2766,12 +2792,12 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     K.tors = tors1;
     K.rec_cap = brenner ? (long)brenner_rec : (long)n * c->prm.bond_rec_avg;
     K.q = dalloc<int>((size_t)K.cap);
-    K.ctr = dalloc<unsigned long long>(4);
+    K.ctr = dalloc<unsigned long long>(3 * kTaskCtr);
     K.rbase = dalloc<long>(n);
     K.nrec = dalloc<int>(n);
     K.rec = dalloc<double>((size_t)K.rec_cap);
     if (!K.q || !K.ctr || !K.rbase || !K.nrec || !K.rec) return fail(MDG_ERR_CUDA, "cudaMalloc (bond tasks)");
-    CK(cudaMemset(K.ctr, 0, 4 * sizeof(unsigned long long)));
+    CK(cudaMemset(K.ctr, 0, 3 * kTaskCtr * sizeof(unsigned long long)));
     int dev = 0, sms = 148, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

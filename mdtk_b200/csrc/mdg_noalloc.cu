@@ -199,16 +199,19 @@ __global__ void k_na_nl(NaView v)
   if (i < v.S.n) nl_build_atom(v.S, v.G, v.L, i, v.status);
 }
 
+constexpr int kNaBondLanes = 8;  // at most 4,096 atoms
 __global__ void k_na_bonds(NaView v, const ReboParams* P)
 {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a < v.S.n) bonds_atom(v.S, v.L, *P, v.BB, a, v.status);
+  const int a = (blockIdx.x * blockDim.x + threadIdx.x) / kNaBondLanes;
+  bonds_atom<kNaBondLanes>(v.S, v.L, *P, v.BB, min(a, v.S.n - 1), a < v.S.n, v.status);
 }
 
 __global__ void k_na_brev(NaView v)
 {
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a < v.S.n) brev_atom(v.BB, a);
+  if (a >= v.S.n) return;
+  const int nb = v.BB.nb[a];
+  for (int s = 0; s < nb; s++) v.BB.brev[a * v.BB.mb + s] = brev_slot(v.BB, a, v.BB.bj[a * v.BB.mb + s]);
 }
 
 __global__ void k_na_rebo(NaView v, const ReboParams* P, const ReboTables* T, TorsParams TP, int do_tors)
@@ -294,7 +297,7 @@ int mdg_rebo_compute_noalloc(int n, const double* pos, const int32_t* z, const d
   const int T = 128, B = (n + T - 1) / T;
   k_na_pack<<<B, T, 0, st>>>(v, pos, z);
   k_na_nl<<<B, T, 0, st>>>(v);
-  k_na_bonds<<<B, T, 0, st>>>(v, s->params);
+  k_na_bonds<<<(n * kNaBondLanes + T - 1) / T, T, 0, st>>>(v, s->params);
   k_na_brev<<<B, T, 0, st>>>(v);
   k_na_rebo<<<B, T, 0, st>>>(v, s->params, s->tables, tp, with_torsion ? 1 : 0);
   k_na_gather<<<B, T, 0, st>>>(v, grad);

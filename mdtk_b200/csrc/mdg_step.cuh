@@ -216,46 +216,77 @@ struct BondBuild {
   double4* nco;
 };
 
+#if defined(__CUDACC__)
 // Bonds of atom a from its REBO-range Verlet list (ascending, as the
 // reference's NL order), with the REBO cutoffs of each pair
-// (REBO::countNeighbours, REBO.cxx:328-393; AtomsPair, AtomsPair.hpp:137-158).
-MDG_HD void bonds_atom(const State& S, const NList& L, const ReboParams& P, BondBuild& B, int a,
-                       unsigned int* status)
+// (REBO::countNeighbours, REBO.cxx:328-393; AtomsPair, AtomsPair.hpp:137-158),
+// on a group of LANES lanes: each takes a list entry, the entries in range
+// keep their order by ballot, and their cutoffs are added in that order.
+// Whole warps call it (live: the lane's atom is real).
+template <int LANES>
+__device__ __forceinline__ void bonds_atom(const State& S, const NList& L, const ReboParams& P, BondBuild& B, int a,
+                                           bool live, unsigned int* status)
 {
+  const int lane = threadIdx.x & 31, gl = lane % LANES, gbase = lane - gl;
+  const unsigned gmask = ((1u << LANES) - 1u) << gbase;
   const double4 pa = S.pos[a];
   const int ta = (int)pa.w;
   const V3 xa = v3(pa.x, pa.y, pa.z);
-  const int cnt = L.cnt[a];
+  const Box box = box_of(S, a);
+  const int cnt = live ? L.cnt[a] : 0;
   const int* lst = L.list + (long)a * L.cap;
+  const int most = __reduce_max_sync(0xffffffffu, cnt);
   double Nt = 0.0, NC = 0.0, NH = 0.0;
   int nb = 0;
-  for (int s = 0; s < cnt; s++) {
-    const int j = lst[s];
-    const double4 pj = S.pos[j];
-    const int tj = (int)pj.w;
-    V3 rv = depos(box_of(S, a), xa, v3(pj.x, pj.y, pj.z));
-    double d2 = norm2(rv);
-    const double R1 = P.R[ta][tj][0], R2 = P.R[ta][tj][1];
-    if (d2 > R2 * R2) continue;
-    double r = sqrt(d2);
-    double f, df;
-    cutoff(r, R1, R2, f, df);
-    double Rp1 = P.Rp[ta][tj][0], Rp2 = P.Rp[ta][tj][1];
-    double fp = Sprime(r, Rp1, Rp2), dfp = dSprime(r, Rp1, Rp2);
-    if (!(r > R2)) {
-      Nt += f;
-      if (tj == kH) NH += f;
-      if (tj == kC) NC += f;
+  for (int base = 0; base < most; base += LANES) {
+    const int s = base + gl;
+    bool in = false;
+    int j = -1, tj = 0;
+    double r = 0.0, f = 0.0, df = 0.0, R1 = 0.0, R2 = 0.0;
+    V3 rv = v3(0, 0, 0);
+    if (s < cnt) {
+      j = lst[s];
+      const double4 pj = S.pos[j];
+      tj = (int)pj.w;
+      rv = depos(box, xa, v3(pj.x, pj.y, pj.z));
+      const double d2 = norm2(rv);
+      R1 = P.R[ta][tj][0];
+      R2 = P.R[ta][tj][1];
+      in = !(d2 > R2 * R2);
+      if (in) {
+        r = sqrt(d2);
+        cutoff(r, R1, R2, f, df);
+      }
     }
-    if (nb < B.mb) {
-      const int q = a * B.mb + nb;
+    unsigned m = __ballot_sync(0xffffffffu, in) & gmask;
+    const int slot = nb + __popc(m & ((1u << lane) - 1u));
+    if (in && slot < B.mb) {
+      const double Rp1 = P.Rp[ta][tj][0], Rp2 = P.Rp[ta][tj][1];
+      const double fp = Sprime(r, Rp1, Rp2), dfp = dSprime(r, Rp1, Rp2);
+      const int q = a * B.mb + slot;
       B.bj[q] = j;
       B.brv[q] = make_double4(rv.x, rv.y, rv.z, r);
       B.bu[q] = make_double4(rv.x / r, rv.y / r, rv.z / r, f);
       B.bd[q] = make_double4(df, fp, dfp, 0.0);
     }
-    nb++;
+    nb += __popc(m);
+    // (a bond counts when its rounded length is within R2, as the reference tests it)
+    const unsigned counts = __ballot_sync(0xffffffffu, in && !(r > R2));
+    const unsigned hyd = __ballot_sync(0xffffffffu, tj == kH), car = __ballot_sync(0xffffffffu, tj == kC);
+    m &= counts;
+    const int n = __reduce_max_sync(0xffffffffu, __popc(m));
+    for (int k = 0; k < n; k++) {
+      const int src = m ? __ffs(m) - 1 : lane;
+      const double fk = __shfl_sync(0xffffffffu, f, src);
+      if (m) {
+        Nt += fk;
+        if (hyd >> src & 1u) NH += fk;
+        if (car >> src & 1u) NC += fk;
+        m &= m - 1;
+      }
+    }
   }
+  if (!live || gl != 0) return;
   if (nb > B.mb) {
     *status |= ST_BOND_OVERFLOW;
     nb = B.mb;
@@ -264,19 +295,15 @@ MDG_HD void bonds_atom(const State& S, const NList& L, const ReboParams& P, Bond
   B.nco[a] = make_double4(Nt, NC, NH, (double)ta);
 }
 
-// Slot of atom a in each partner's bond list.
-MDG_HD void brev_atom(BondBuild& B, int a)
+// Slot of atom a in the list of its partner j (-1: not there).
+__device__ __forceinline__ int brev_slot(const BondBuild& B, int a, int j)
 {
-  const int nb = B.nb[a];
-  for (int s = 0; s < nb; s++) {
-    const int j = B.bj[a * B.mb + s];
-    const int nbj = B.nb[j];
-    int r = -1;
-    for (int t = 0; t < nbj; t++)
-      if (B.bj[j * B.mb + t] == a) { r = t; break; }
-    B.brev[a * B.mb + s] = r;
-  }
+  const int nbj = B.nb[j];
+  for (int t = 0; t < nbj; t++)
+    if (B.bj[j * B.mb + t] == a) return t;
+  return -1;
 }
+#endif
 
 // Per-atom force-evaluation outputs (W: double, or dual on the adjoint path).
 template <class Ws>
@@ -338,6 +365,7 @@ MDG_HD void rebo_atom(const ReboT<Real, TB>& R, const TorsParams& TP, int do_reb
 // an atom's slots lie consecutively from rbase[a]; a per-atom reduction sums
 // them in slot order.  Splitting an atom's bonds over threads shortens the
 // longest serial chain from all of a carbon's bonds to one bond.
+constexpr int kTaskCtr = 16;
 struct BondTasks {
   int cap;                  // queue capacity (n * mb)
   // 0: one task per directed slot; 1: one task per bond (slots to higher
@@ -346,7 +374,8 @@ struct BondTasks {
   int pairs;
   int tors;                 // torsion on (mode 2 gives C-C bonds a torsion record at each end)
   int* q;                   // slots a*mb+s: C-C bonds from the front, the rest from the back
-  unsigned long long* ctr;  // [0] C-C tasks, [1] other tasks, [2] record doubles handed out
+  unsigned long long* ctr;  // C-C tasks, other tasks, record doubles handed out, at ctr[k kTaskCtr]
+                            // (one 128-byte line each)
   long* rbase;              // [n] first record double of atom a (-1: over capacity, flagged)
   int* nrec;                // [n] records of atom a: its bond slots, then (mode 2) its C-C torsion records
   double* rec;
