@@ -3048,14 +3048,22 @@ int mdg_nl_pairs(mdg_ctx* c, int list_id, int32_t* pairs, int64_t cap, int64_t* 
 // given split.
 // Time one force evaluation as the steps run it: captured into a CUDA graph
 // (stream overlap and dependent launches included) and replayed four times
-// back to back per sample; the best of three samples, per evaluation.
+// back to back per sample; the best of three samples, per evaluation.  Where
+// the accelerations are yet to be set (init_first_step follows), it is a whole
+// step of dt 0, which leaves the positions and velocities as they are: two
+// configurations whose bare evaluations differ by 0.1% took 273 and 286 us a
+// step on 43,680 ethane atoms.
 static int time_eval_graph(mdg_ctx* c, cudaEvent_t e0, cudaEvent_t e1, float* best)
 {
+  StepDev still;
+  std::memset(&still, 0, sizeof(still));
+  still.nlc0 = c->nl[0].cnt;
+  const bool step = !c->acc_valid && !c->snap;
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ge = nullptr;
   const int64_t l0 = c->launches;
   CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = evaluate(c);
+  int rc = evaluate(c, step ? &still : nullptr);
   cudaError_t ce = cudaStreamEndCapture(c->stream, &g);
   c->launches = l0;
   if (rc) {
