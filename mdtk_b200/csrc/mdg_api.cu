@@ -1757,7 +1757,7 @@ struct mdg_ctx {
   // connectivity kernels
   bool overlap = false;
   cudaStream_t side = nullptr, side2 = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork2 = nullptr, ev_join2 = nullptr;
+  cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_fork2 = nullptr, ev_join2 = nullptr, ev_join3 = nullptr;
   int* lj_inr = nullptr;      // [n * LJ list cap] in-range LJ partners of the step: far from the front, close from the back
   int* lj_inr_cnt = nullptr;  // [2n] far counts, close counts
   bool tuned = false;        // the autotuner ran for this system
@@ -2216,6 +2216,17 @@ int rebuild_lists(mdg_ctx* c, const StepDev* step = nullptr)
   return launch_check(c);
 }
 
+// The embedding, pair and ion terms of the metal list, on stream st.
+int metal_terms(mdg_ctx* c, cudaStream_t st)
+{
+  State S = c->S();
+  LAUNCH_ON(c, st, "eam_density", k_eam_rho, nblk(c->n * 32), kThreads, S, c->nl[2], c->d_metal, c->d_fp, c->d_em,
+            c->d_status);
+  LAUNCH_ON(c, st, "metal_pairs", k_metal_pairs, nblk(c->n * 32), kThreads, S, c->nl[2], c->d_metal, c->d_fp, c->d_em,
+            c->d_gm);
+  return MDG_OK;
+}
+
 // One force evaluation at the current positions; leaves dE/dx in c->grad and
 // per-atom energies in c->fo.  With a step, the evaluation is the body of a
 // velocity-Verlet step: the position update comes first (fused with the
@@ -2246,8 +2257,16 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
     LAUNCH_ON(c, c->side2, "lj_filter", k_lj_filter, std::min(nblk(c->n * 32), c->warp_blocks), kThreads, c->ljp, S,
               c->ljt, c->lj_inr, c->lj_inr_cnt, c->lj_inr_cnt + c->n);
     CK(cudaEventRecord(c->ev_join2, c->side2));
+    if (c->has_list[2]) {
+      // the metal and ion terms need positions only: beside the hydrocarbons,
+      // behind the filter (19,233 atoms of a Cu slab: 203 us a step with them
+      // in the main chain, 190 so)
+      rc = rebuild_list(c, 2, c->side2);
+      if (!rc) rc = metal_terms(c, c->side2);
+      if (rc) return rc;
+      CK(cudaEventRecord(c->ev_join3, c->side2));
+    }
     rc = rebuild_list(c, 0, c->stream);
-    if (!rc) rc = rebuild_list(c, 2, c->stream);
     if (rc) return rc;
   } else {
     rc = rebuild_lists(c, step);
@@ -2357,10 +2376,12 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
            tasks ? 1 : 0, c->spc, lj ? 1 : 0, c->fo);
   }
   if (c->has_list[2]) {
-    LAUNCH(c, "eam_density", k_eam_rho, nblk(c->n * 32), kThreads, S, c->nl[2], c->d_metal, c->d_fp, c->d_em,
-           c->d_status);
-    LAUNCH(c, "metal_pairs", k_metal_pairs, nblk(c->n * 32), kThreads, S, c->nl[2], c->d_metal, c->d_fp, c->d_em,
-           c->d_gm);
+    if (ovl) {
+      CK(cudaStreamWaitEvent(c->stream, c->ev_join3, 0));
+    } else {
+      rc = metal_terms(c, c->stream);
+      if (rc) return rc;
+    }
   }
   if (step) {
     LAUNCH(c, "gather_verlet_vel", k_gather_vv, nblk(c->n * kGatherLanes), kThreads, B, c->fo, lj ? 1 : 0, c->spc, c->grad, S,
@@ -2510,7 +2531,8 @@ int mdg_create(const mdg_params* p, mdg_ctx** out)
       cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork2, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess) {
     mdg_destroy(c);
     return fail(MDG_ERR_CUDA, "cudaStreamCreate / cudaEventCreate");
   }
@@ -2552,6 +2574,7 @@ int mdg_destroy(mdg_ctx* c)
   if (c->ev_join) cudaEventDestroy(c->ev_join);
   if (c->ev_fork2) cudaEventDestroy(c->ev_fork2);
   if (c->ev_join2) cudaEventDestroy(c->ev_join2);
+  if (c->ev_join3) cudaEventDestroy(c->ev_join3);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->side2) cudaStreamDestroy(c->side2);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);

@@ -39,6 +39,8 @@ struct MetalParams {
   double ack_x[2];                   // Ackland joining cubic interval (cm)
   double ack_v[3][3][4];
   double rcut;                       // largest range of the three (cm)
+  double range2[kNSpec][kNSpec];     // squared range of each species pair (A^2): beyond it every term is 0
+  double rho2[3][3];                 // squared range of the density (A^2)
 };
 
 // Ziegler-Biersack-Littmark universal screened Coulomb repulsion with the
@@ -256,6 +258,19 @@ inline void make_metal_params(MetalParams& M)
       v[0] = zbl(M.Z[kCu + a], M.Z[kCu + b], M.ack_x[0], v[1]);
       v[2] = ack_knots(M, a, b, a == b, M.ack_x[1], v[3]);
     }
+  // (a part in 1e12 above the ranges: rounding never leaves a pair out)
+  const double over = 1.0 + 1e-12;
+  for (int a = 0; a < kNSpec; a++)
+    for (int b = 0; b < kNSpec; b++) {
+      double r = M.rcut;
+      if (spec_metal(a) && spec_metal(b)) {
+        const int x = a - kCu, y = b - kCu;
+        const double g = std::fmin(M.Rk[x][x][1], M.Rk[y][y][1]);
+        r = std::fmax(M.rk[x][y][1], g);
+        M.rho2[x][y] = g / Ao * (g / Ao) * over;
+      }
+      M.range2[a][b] = r / Ao * (r / Ao) * over;
+    }
 }
 
 MDG_HD double warp_sum(double x)
@@ -267,13 +282,13 @@ MDG_HD double warp_sum(double x)
 }
 
 // The partners of atom i within the potentials' range, handed to the lanes
-// 32 at a time: each lane tests one list entry, a ballot packs the ones in
-// range into a per-warp queue in list order, and every full queue is
+// 32 at a time: each lane tests one list entry against its species' range
+// (range2), a ballot packs the ones in range into a per-warp queue in list order, and every full queue is
 // processed with all lanes busy (two thirds of a Verlet list lie in its
 // skin).  f(j, lane) is called once per queued partner; deterministic.
 template <class F>
-__device__ void for_partners(const State& S, const NList& L, int i, const V3& xi, const Box& box, double rcut_A,
-                             bool metal_only, int* wq, F&& f)
+__device__ void for_partners(const State& S, const NList& L, int i, const V3& xi, const Box& box,
+                             const double* range2, int* wq, F&& f)
 {
   const int lane = threadIdx.x & 31;
   const int* nl = L.list + (long)i * L.cap;
@@ -286,7 +301,7 @@ __device__ void for_partners(const State& S, const NList& L, int i, const V3& xi
     if (q < nn) {
       j = nl[q];
       const double4 pj = S.pos[j];
-      if (!metal_only || spec_metal((int)pj.w)) keep = norm2(depos(box, xi, v3(pj.x, pj.y, pj.z))) < rcut_A * rcut_A;
+      keep = norm2(depos(box, xi, v3(pj.x, pj.y, pj.z))) < range2[(int)pj.w];
     }
     const unsigned m = __ballot_sync(0xffffffffu, keep);
     const int pos = cnt + __popc(m & ((1u << lane) - 1u));
@@ -338,7 +353,9 @@ __global__ void k_eam_rho(State S, NList L, const MetalParams* __restrict__ Mp, 
     const double4 pj = S.pos[nl[q]];
     const int tj = (int)pj.w;
     if (!spec_metal(tj)) continue;
-    const double r = sqrt(norm2(depos(box, xi, v3(pj.x, pj.y, pj.z)))) * kAo;
+    const double d2 = norm2(depos(box, xi, v3(pj.x, pj.y, pj.z)));
+    if (d2 >= M.rho2[ti - kCu][tj - kCu]) continue;
+    const double r = sqrt(d2) * kAo;
     double d;
     rho += ack_g(M, ti - kCu, tj - kCu, r, d);
   }
@@ -369,7 +386,7 @@ __global__ void k_metal_pairs(State S, NList L, const MetalParams* __restrict__ 
   const V3 xi = v3(pi.x, pi.y, pi.z);
   const double fpi = fp[i];
   double e = 0.0, gx = 0.0, gy = 0.0, gz = 0.0;
-  for_partners(S, L, i, xi, box, M.rcut / kAo, false, qbuf + (threadIdx.x & ~31), [&](int j) {
+  for_partners(S, L, i, xi, box, M.range2[ti], qbuf + (threadIdx.x & ~31), [&](int j) {
     const double4 pj = S.pos[j];
     const int tj = (int)pj.w;
     const V3 d = depos(box, xi, v3(pj.x, pj.y, pj.z));
