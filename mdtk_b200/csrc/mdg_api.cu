@@ -43,6 +43,10 @@ int fail(int code, const std::string& msg)
   } while (0)
 
 constexpr int kThreads = 128;
+// States up to this size pass through the context's pinned memory in one copy;
+// larger ones go straight between the device and the caller's arrays (pinned
+// callers keep their DMA).
+constexpr size_t kStagedBytes = 256 * 1024;
 constexpr int kRedBlocks = 296;  // two per SM
 constexpr double kAo = 1e-8, kEv = 1.6021e-12, kFs = 1e-15;
 
@@ -238,7 +242,7 @@ __device__ void block_alloc3(const unsigned long long v[3], unsigned long long* 
     if (lane == 31) ws[k][wid] = x[k];
   }
   __syncthreads();
-  if (threadIdx.x < 3) {
+  if (threadIdx.x < N) {
     const int k = threadIdx.x;
     unsigned long long run = 0;
     for (int w = 0; w < NT / 32; w++) {
@@ -250,7 +254,7 @@ __device__ void block_alloc3(const unsigned long long v[3], unsigned long long* 
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < 3; k++) out[k] = base[k] + ws[k][wid] + x[k] - v[k];
+  for (int k = 0; k < N; k++) out[k] = base[k] + ws[k][wid] + x[k] - v[k];
 }
 
 // Reverse slots, then the REBO bond tasks of each atom: record space and the
@@ -1472,11 +1476,46 @@ __global__ void k_state_unpack(State S, const double* io, double ul, double uv)
   S.pos[i] = make_double4(p[0] * ul, p[1] * ul, p[2] * ul, S.pos[i].w);
   S.vel[i] = make_double4(v[0] * uv, v[1] * uv, v[2] * uv, 0.0);
 }
-__global__ void k_state_pack(State S, double* io, double ul, double uv)
+// mdg_set_state: as k_state_unpack, with the positions wrapped into the box
+// (Atom::applyPBC; the host has checked them) and their periods counted.
+__global__ void k_state_set(State S, const double* io, double ul, double uv, int with_vel)
 {
   pdl_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= S.n) return;
+  const double* p = io + 3 * (long)i;
+  double x[3] = {p[0] * ul, p[1] * ul, p[2] * ul};
+  const int4 im0 = S.image[i];
+  int im[3] = {im0.x, im0.y, im0.z};
+  const Box box = box_of(S, i);
+#pragma unroll
+  for (int a = 0; a < 3; a++)
+    if (box.pbc[a] && (x[a] < 0 || x[a] >= box.L[a])) {
+      // (rounded as the host's wrap1: no contraction)
+      const double nsh = floor(x[a] / box.L[a]);
+      x[a] = __dsub_rn(x[a], __dmul_rn(nsh, box.L[a]));
+      im[a] += (int)nsh;
+      for (int q = 0; q < 2 && x[a] < 0; q++) { x[a] += box.L[a]; --im[a]; }
+      for (int q = 0; q < 2 && x[a] >= box.L[a]; q++) { x[a] -= box.L[a]; ++im[a]; }
+    }
+  S.pos[i] = make_double4(x[0], x[1], x[2], S.pos[i].w);
+  S.image[i] = make_int4(im[0], im[1], im[2], 0);
+  if (with_vel) {
+    const double* v = io + 3 * ((long)S.n + i);
+    S.vel[i] = make_double4(v[0] * uv, v[1] * uv, v[2] * uv, 0.0);
+  }
+}
+// (images, when asked for, follow the 6 n doubles as [n*3] int32)
+__global__ void k_state_pack(State S, double* io, double ul, double uv, int images)
+{
+  pdl_enter();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= S.n) return;
+  if (images) {
+    int* m = reinterpret_cast<int*>(io + 6 * (long)S.n) + 3 * (long)i;
+    const int4 im = S.image[i];
+    m[0] = im.x; m[1] = im.y; m[2] = im.z;
+  }
   const double4 p = S.pos[i], v = S.vel[i];
   double* po = io + 3 * (long)i;
   double* vo = io + 3 * ((long)S.n + i);
@@ -1822,8 +1861,11 @@ struct mdg_ctx {
   size_t ev_used = 0;
   std::vector<std::pair<std::string, size_t>> prof_recs;  // name, index of the start event
   // host staging for mdg_step_host
-  double4* h_stage = nullptr;
-  double* d_io = nullptr;       // [6 n] the host step's pos and vel in the caller's [n*3] layout
+  double* h_stage = nullptr;    // [8 n] pinned: states and gradients on their way between caller and device
+  bool stage_busy = false;      // an upload may still be reading it (until ev_stage)
+  cudaEvent_t ev_stage = nullptr;
+  double* h_small = nullptr;    // [8] pinned: energies (0-3), the status word (7)
+  double* d_io = nullptr;       // [8 n] pos, vel and image counters in the caller's [n*3] layout
   std::vector<int> h_type;
   AdjWs* adj = nullptr;       // adjoint path, allocated on first use
 
@@ -1996,6 +2038,8 @@ void free_system(mdg_ctx* c)
   for (void* p : bq)
     if (p) cudaFree(p);
   std::memset(&c->bt, 0, sizeof(c->bt));
+  if (c->stage_busy) cudaEventSynchronize(c->ev_stage);
+  c->stage_busy = false;
   if (c->h_stage) cudaFreeHost(c->h_stage);
   c->h_stage = nullptr;
   if (c->h_elog) cudaFreeHost(c->h_elog);
@@ -2422,11 +2466,15 @@ int reduce_energies(mdg_ctx* c, double* out_dev, int* log_row, bool with_kin, bo
   return launch_check(c);
 }
 
+// Waits for the stream (and every copy queued on it) and reports the device's
+// status word.
 int read_status(mdg_ctx* c)
 {
-  unsigned int st = 0;
-  CK(cudaMemcpyAsync(&st, c->d_status, sizeof(st), cudaMemcpyDeviceToHost, c->stream));
+  unsigned int* h = reinterpret_cast<unsigned int*>(c->h_small + 7);
+  CK(cudaMemcpyAsync(h, c->d_status, sizeof(*h), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  c->stage_busy = false;
+  const unsigned int st = *h;
   if (st) {
     unsigned int z = 0;
     CK(cudaMemcpy(c->d_status, &z, sizeof(z), cudaMemcpyHostToDevice));
@@ -2434,6 +2482,14 @@ int read_status(mdg_ctx* c)
     int code = status_to_code(st, msg);
     return fail(code, msg);
   }
+  return MDG_OK;
+}
+
+// Before the host writes h_stage again.
+int stage_wait(mdg_ctx* c)
+{
+  if (c->stage_busy) CK(cudaEventSynchronize(c->ev_stage));
+  c->stage_busy = false;
   return MDG_OK;
 }
 
@@ -2532,7 +2588,9 @@ int mdg_create(const mdg_params* p, mdg_ctx** out)
       cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_fork2, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->ev_join2, cudaEventDisableTiming) != cudaSuccess ||
-      cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess) {
+      cudaEventCreateWithFlags(&c->ev_join3, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&c->ev_stage, cudaEventDisableTiming) != cudaSuccess ||
+      cudaHostAlloc((void**)&c->h_small, 8 * sizeof(double), cudaHostAllocDefault) != cudaSuccess) {
     mdg_destroy(c);
     return fail(MDG_ERR_CUDA, "cudaStreamCreate / cudaEventCreate");
   }
@@ -2575,6 +2633,8 @@ int mdg_destroy(mdg_ctx* c)
   if (c->ev_fork2) cudaEventDestroy(c->ev_fork2);
   if (c->ev_join2) cudaEventDestroy(c->ev_join2);
   if (c->ev_join3) cudaEventDestroy(c->ev_join3);
+  if (c->ev_stage) cudaEventDestroy(c->ev_stage);
+  if (c->h_small) cudaFreeHost(c->h_small);
   if (c->side) cudaStreamDestroy(c->side);
   if (c->side2) cudaStreamDestroy(c->side2);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
@@ -2585,7 +2645,10 @@ int mdg_destroy(mdg_ctx* c)
 int mdg_set_stream(mdg_ctx* c, void* stream)
 {
   if (!c) return fail(MDG_ERR_ARG, "null context");
-  c->stream = stream ? (cudaStream_t)stream : c->own_stream;
+  cudaStream_t next = stream ? (cudaStream_t)stream : c->own_stream;
+  // a state on its way to the device is not left behind on the old stream
+  if (next != c->stream && c->stage_busy) CK(cudaStreamSynchronize(c->stream));
+  c->stream = next;
   return MDG_OK;
 }
 
@@ -2874,9 +2937,9 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     c->cij_scratch = dalloc<int>((size_t)c->cij_blocks * kCijAtoms * kCijScratch);
     if (!c->cij_scratch) return fail(MDG_ERR_CUDA, "cudaMalloc (connectivity)");
   }
-  if (cudaHostAlloc((void**)&c->h_stage, 2 * (size_t)n * sizeof(double4), cudaHostAllocDefault) != cudaSuccess)
+  if (cudaHostAlloc((void**)&c->h_stage, 8 * (size_t)n * sizeof(double), cudaHostAllocDefault) != cudaSuccess)
     return fail(MDG_ERR_CUDA, "cudaHostAlloc (staging)");
-  c->d_io = dalloc<double>(6 * (size_t)n);
+  c->d_io = dalloc<double>(8 * (size_t)n);
   if (!c->d_io) return fail(MDG_ERR_CUDA, "cudaMalloc (host-step staging)");
   // per-system step state: bath temperature, adaptive dt, time, v_max
   c->d_tb_T = dalloc<double>(nsys);
@@ -2947,35 +3010,29 @@ int mdg_set_state(mdg_ctx* c, const double* pos, const double* vel)
 {
   if (!c || !c->n) return fail(MDG_ERR_STATE, "no system loaded");
   const int n = c->n;
-  std::vector<double4> hp(n), hv;
-  std::vector<int4> him(n);
-  std::vector<double4> old(n);
-  CK(cudaMemcpyAsync(old.data(), c->pos, n * sizeof(double4), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(him.data(), c->image, n * sizeof(int4), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaStreamSynchronize(c->stream));
+  int rc = stage_wait(c);
+  if (rc) return rc;
+  // checked here and copied to pinned memory as they are; the device converts
+  // and wraps them, so nothing has to come back from it first
+  double* h = c->h_stage;
   for (int i = 0; i < n; i++) {
-    double x[3];
-    int im[3] = {him[i].x, him[i].y, him[i].z};
+    const Box& bx = c->h_boxes[c->h_sys[i]];
     for (int a = 0; a < 3; a++) {
-      x[a] = pos[3 * i + a] * c->unit_len;
-      if (!std::isfinite(x[a])) return fail(MDG_ERR_NONFINITE, "non-finite coordinate");
-      const Box& bx = c->h_boxes[c->h_sys[i]];
-      if (bx.pbc[a] && !wrap1(x[a], im[a], bx.L[a])) return fail(MDG_ERR_ARG, "coordinate too far outside the box");
+      const double x = pos[3 * i + a] * c->unit_len;
+      if (!std::isfinite(x)) return fail(MDG_ERR_NONFINITE, "non-finite coordinate");
+      if (bx.pbc[a] && (x < 0 || x >= bx.L[a]) && std::fabs(std::floor(x / bx.L[a])) > 1e9)
+        return fail(MDG_ERR_ARG, "coordinate too far outside the box");
+      h[3 * i + a] = pos[3 * i + a];
     }
-    hp[i] = make_double4(x[0], x[1], x[2], old[i].w);
-    him[i] = make_int4(im[0], im[1], im[2], 0);
   }
-  CK(cudaMemcpyAsync(c->pos, hp.data(), n * sizeof(double4), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(c->image, him.data(), n * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
-  if (vel) {
-    hv.resize(n);
-    for (int i = 0; i < n; i++)
-      hv[i] = make_double4(vel[3 * i] * c->unit_vel, vel[3 * i + 1] * c->unit_vel, vel[3 * i + 2] * c->unit_vel, 0.0);
-    CK(cudaMemcpyAsync(c->vel, hv.data(), n * sizeof(double4), cudaMemcpyHostToDevice, c->stream));
-  }
-  CK(cudaStreamSynchronize(c->stream));
+  if (vel) std::memcpy(h + 3 * (size_t)n, vel, 3 * (size_t)n * sizeof(double));
+  CK(cudaMemcpyAsync(c->d_io, h, (vel ? 6 : 3) * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  State S = c->S();
+  LAUNCH(c, "state_set", k_state_set, nblk(n), kThreads, S, c->d_io, c->unit_len, c->unit_vel, vel ? 1 : 0);
+  CK(cudaEventRecord(c->ev_stage, c->stream));
+  c->stage_busy = true;
   c->acc_valid = false;
-  return MDG_OK;
+  return launch_check(c);
 }
 
 int mdg_compute(mdg_ctx* c, double* e_total, double* e_terms, double* grad)
@@ -2985,13 +3042,12 @@ int mdg_compute(mdg_ctx* c, double* e_total, double* e_terms, double* grad)
   if (rc) return rc;
   rc = reduce_energies(c, c->d_energy, nullptr, false, true, c->grad);
   if (rc) return rc;
-  double he[4] = {0, 0, 0, 0};
+  double* he = c->h_small;
+  he[3] = 0.0;
   CK(cudaMemcpyAsync(he, c->d_energy, (c->has_list[2] ? 4 : 3) * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  std::vector<double4> hg;
-  if (grad) {
-    hg.resize(c->n);
-    CK(cudaMemcpyAsync(hg.data(), c->grad, c->n * sizeof(double4), cudaMemcpyDeviceToHost, c->stream));
-  }
+  const double4* hg = reinterpret_cast<const double4*>(c->h_stage);
+  if (grad)
+    CK(cudaMemcpyAsync(c->h_stage, c->grad, c->n * sizeof(double4), cudaMemcpyDeviceToHost, c->stream));
   rc = read_status(c);
   if (rc) return rc;
   double E = (he[0] + he[1]) + he[2];
@@ -3541,19 +3597,26 @@ int mdg_get_state(mdg_ctx* c, double* pos, double* vel, int32_t* image)
 {
   if (!c || !c->n) return fail(MDG_ERR_STATE, "no system loaded");
   const int n = c->n;
-  std::vector<double4> hp(n), hv(n);
-  std::vector<int4> him(n);
-  CK(cudaMemcpyAsync(hp.data(), c->pos, n * sizeof(double4), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(hv.data(), c->vel, n * sizeof(double4), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(him.data(), c->image, n * sizeof(int4), cudaMemcpyDeviceToHost, c->stream));
-  int rc = read_status(c);
-  if (rc) return rc;
-  for (int i = 0; i < n; i++) {
-    if (pos) { pos[3*i] = hp[i].x / c->unit_len; pos[3*i+1] = hp[i].y / c->unit_len; pos[3*i+2] = hp[i].z / c->unit_len; }
-    if (vel) { vel[3*i] = hv[i].x / c->unit_vel; vel[3*i+1] = hv[i].y / c->unit_vel; vel[3*i+2] = hv[i].z / c->unit_vel; }
-    if (image) { image[3*i] = him[i].x; image[3*i+1] = him[i].y; image[3*i+2] = him[i].z; }
+  const size_t bytes = 3 * (size_t)n * sizeof(double);
+  // packed into the caller's layout on the device
+  State S = c->S();
+  double* io = c->d_io;
+  LAUNCH(c, "state_pack", k_state_pack, nblk(n), kThreads, S, io, c->unit_len, c->unit_vel, image ? 1 : 0);
+  if (8 * (size_t)n * sizeof(double) <= kStagedBytes) {
+    // small: one copy to pinned memory, one wait
+    CK(cudaMemcpyAsync(c->h_stage, io, 8 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    int rc = read_status(c);
+    if (rc) return rc;
+    if (pos) std::memcpy(pos, c->h_stage, bytes);
+    if (vel) std::memcpy(vel, c->h_stage + 3 * (size_t)n, bytes);
+    if (image) std::memcpy(image, c->h_stage + 6 * (size_t)n, 3 * (size_t)n * sizeof(int32_t));
+    return MDG_OK;
   }
-  return MDG_OK;
+  if (pos) CK(cudaMemcpyAsync(pos, io, bytes, cudaMemcpyDeviceToHost, c->stream));
+  if (vel) CK(cudaMemcpyAsync(vel, io + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost, c->stream));
+  if (image)
+    CK(cudaMemcpyAsync(image, io + 6 * (size_t)n, 3 * (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
+  return read_status(c);
 }
 
 int64_t mdg_launch_count(mdg_ctx* c) { return c ? c->launches : 0; }
@@ -3607,18 +3670,38 @@ int mdg_step_host(mdg_ctx* c, int nsteps, double dt, double* pos, double* vel, d
   // straight from and to them when they are pinned) and are converted to and
   // from the device layout by kernels
   double* io = c->d_io;
-  CK(cudaMemcpyAsync(io, pos, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
-  CK(cudaMemcpyAsync(io + 3 * (size_t)n, vel, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, c->stream));
+  const size_t bytes = 3 * (size_t)n * sizeof(double);
+  const bool staged = 2 * bytes <= kStagedBytes;  // small states go through pinned memory, one copy each way
+  if (staged) {
+    int rc = stage_wait(c);
+    if (rc) return rc;
+    std::memcpy(c->h_stage, pos, bytes);
+    std::memcpy(c->h_stage + 3 * (size_t)n, vel, bytes);
+    CK(cudaMemcpyAsync(io, c->h_stage, 2 * bytes, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaEventRecord(c->ev_stage, c->stream));
+    c->stage_busy = true;
+  } else {
+    CK(cudaMemcpyAsync(io, pos, bytes, cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(io + 3 * (size_t)n, vel, bytes, cudaMemcpyHostToDevice, c->stream));
+  }
   State S = c->S();
   LAUNCH(c, "state_unpack", k_state_unpack, nblk(n), kThreads, S, io, c->unit_len, c->unit_vel);
   // one synchronisation for the whole call: the energy log, the state and
   // the status come back together
   int rc = run_steps(c, nsteps, dt, epot, etot, true, true);
   if (rc) return rc;
-  LAUNCH(c, "state_pack", k_state_pack, nblk(n), kThreads, S, io, c->unit_len, c->unit_vel);
-  CK(cudaMemcpyAsync(pos, io, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-  CK(cudaMemcpyAsync(vel, io + 3 * (size_t)n, 3 * (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+  LAUNCH(c, "state_pack", k_state_pack, nblk(n), kThreads, S, io, c->unit_len, c->unit_vel, 0);
+  if (staged) {
+    CK(cudaMemcpyAsync(c->h_stage, io, 2 * bytes, cudaMemcpyDeviceToHost, c->stream));
+  } else {
+    CK(cudaMemcpyAsync(pos, io, bytes, cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(vel, io + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost, c->stream));
+  }
   rc = read_status(c);
+  if (staged) {
+    std::memcpy(pos, c->h_stage, bytes);
+    std::memcpy(vel, c->h_stage + 3 * (size_t)n, bytes);
+  }
   if (rc) return rc;
   if (epot || etot) fill_energy_log(c, nsteps, epot, etot);
   return MDG_OK;
