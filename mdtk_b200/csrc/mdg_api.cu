@@ -242,7 +242,7 @@ __device__ void block_alloc3(const unsigned long long v[3], unsigned long long* 
     if (lane == 31) ws[k][wid] = x[k];
   }
   __syncthreads();
-  if (threadIdx.x < N) {
+  if (threadIdx.x < 3) {
     const int k = threadIdx.x;
     unsigned long long run = 0;
     for (int w = 0; w < NT / 32; w++) {
@@ -254,7 +254,7 @@ __device__ void block_alloc3(const unsigned long long v[3], unsigned long long* 
   }
   __syncthreads();
 #pragma unroll
-  for (int k = 0; k < N; k++) out[k] = base[k] + ws[k][wid] + x[k] - v[k];
+  for (int k = 0; k < 3; k++) out[k] = base[k] + ws[k][wid] + x[k] - v[k];
 }
 
 // Reverse slots, then the REBO bond tasks of each atom: record space and the
