@@ -432,8 +432,8 @@ __device__ Real baver_end(const ReboT<Real, TB>& R, int e, int i, int j, const P
   const Real sother = pair_swap(smine, pm);
   const Real s1 = is_ci ? smine : sother, s2 = is_ci ? sother : smine;
   Real Nconj = 1.0;
-  Nconj += SQR(s1);
-  Nconj += SQR(s2);
+  add_prod(Nconj, s1, s1);
+  add_prod(Nconj, s2, s2);
   Real F[4];
   t_eval(R.T, fam, Nti, Ntj, Nconj, F, R.status);
   val += F[0];

@@ -103,6 +103,16 @@ struct SinkT {
 };
 typedef SinkT<double> Sink;
 
+// s += a b.  In double each operation is rounded on its own, so that N^conj,
+// whose last bit the pi^rc cells' monomials magnify a million times, is the
+// same number in every kernel (and the reference's).
+template <class Real>
+MDG_HD void add_prod(Real& s, Real a, Real b)
+{
+  if constexpr (std::is_same<Real, double>::value) s = add_rn(s, mul_rn(a, b));
+  else s += a * b;
+}
+
 // Both ends of a bond (lo, hi) at once: contributions are routed to each
 // end's record exactly as two single-end Sinks would route them (the same
 // additions in the same order), so one evaluation of the bond replaces two.
@@ -417,7 +427,7 @@ struct ReboT {
       if (k == o || type(k) != kC) continue;
       Real f = ld(&B.bu[q].w);
       Real N = Nk_excl(k, ld(&B.brv[q].w), f, c);
-      sum += f * Sprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1]));
+      add_prod(sum, f, Sprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1])));
     }
     return sum;
   }
@@ -457,8 +467,8 @@ struct ReboT {
     s1 = nconj_sum(i, j);
     s2 = nconj_sum(j, i);
     Real N = 1.0;
-    N += SQR(s1);
-    N += SQR(s2);
+    add_prod(N, s1, s1);
+    add_prod(N, s2, s2);
     return N;
   }
   template <class S>
