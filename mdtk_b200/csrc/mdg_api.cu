@@ -1150,7 +1150,7 @@ __device__ __forceinline__ void lj_pairs_block(const LJParams& P, const CijTable
       if constexpr (std::is_same<Real, double>::value)
         kind = lj_far_pair(P, T, S, a, b, xa, ta, box, amask, sk.g, e);
       else
-        kind = lj_plain_pair<Real>(P, T, S, a, b, xa, ta, amask, sk, e, nullptr, true);
+        kind = lj_far_pair_f32(P, T, S, a, b, xa, ta, box, amask, sk.g, e);
     }
     note(kind == 2, b);
   }
