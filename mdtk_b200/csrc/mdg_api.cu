@@ -193,6 +193,59 @@ __global__ void k_cell_sort(Grid g, const int* need)
   g.ccursor[c] = 0;
 }
 
+// The four kernels above in one block, for systems of up to kOneBlockAtoms
+// atoms and kOneBlockCells cells.  A step launches them whether a rebuild is due
+// or not, and a kernel that returns at once still costs 2 us of the step's
+// chain; one block takes about CELLS_US us for the rebuild of 43,680 atoms, due
+// every ~30 steps, and beyond these sizes that outweighs the launches.
+constexpr int kOneBlockAtoms = 65536, kOneBlockCells = 262144, kOneBlockThreads = 1024;
+__global__ void __launch_bounds__(kOneBlockThreads) k_cells(State S, Grid g, const int* need)
+{
+  pdl_enter();
+  if (!*need) return;
+  __shared__ int wsum[kOneBlockThreads / 32];
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+  for (int i = t; i < S.n; i += kOneBlockThreads) atomicAdd(&g.ccount[cell_of(g, S, i)], 1);
+  __threadfence();
+  __syncthreads();
+  // exclusive scan of the counts, a tile of one cell a thread at a time
+  int carry = 0;  // the same in every thread
+  for (int b = 0; b < g.ncell; b += kOneBlockThreads) {
+    const int v = b + t < g.ncell ? __ldcg(&g.ccount[b + t]) : 0;
+    int x = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (lane == 31) wsum[wid] = x;
+    __syncthreads();
+    int before = 0, total = 0;
+    for (int w = 0; w < kOneBlockThreads / 32; w++) {
+      const int s = wsum[w];
+      if (w < wid) before += s;
+      total += s;
+    }
+    if (b + t < g.ncell) g.cstart[b + t] = carry + before + x - v;
+    carry += total;
+    __syncthreads();
+  }
+  if (t == 0) g.cstart[g.ncell] = carry;
+  __threadfence();
+  __syncthreads();
+  for (int i = t; i < S.n; i += kOneBlockThreads) {
+    const int c = cell_of(g, S, i);
+    g.catoms[__ldcg(&g.cstart[c]) + atomicAdd(&g.ccursor[c], 1)] = i;
+  }
+  __threadfence();
+  __syncthreads();
+  for (int c = t; c < g.ncell; c += kOneBlockThreads) {
+    const int b = __ldcg(&g.cstart[c]), e = __ldcg(&g.cstart[c + 1]);
+    isort(g.catoms + b, e - b);
+    g.ccount[c] = 0;
+    g.ccursor[c] = 0;
+  }
+}
+
 __global__ void k_nl_build(State S, Grid g, NList L, const int* need, unsigned int* status)
 {
   pdl_enter();
@@ -432,8 +485,8 @@ __device__ Real baver_end(const ReboT<Real, TB>& R, int e, int i, int j, const P
   const Real sother = pair_swap(smine, pm);
   const Real s1 = is_ci ? smine : sother, s2 = is_ci ? sother : smine;
   Real Nconj = 1.0;
-  add_prod(Nconj, s1, s1);
-  add_prod(Nconj, s2, s2);
+  add_prod<true>(Nconj, s1, s1);
+  add_prod<true>(Nconj, s2, s2);
   Real F[4];
   t_eval(R.T, fam, Nti, Ntj, Nconj, F, R.status);
   val += F[0];
@@ -2236,7 +2289,9 @@ int rebuild_list(mdg_ctx* c, int l, cudaStream_t st)
   NList& L = c->nl[l];
   Grid& g = c->grid[l];
   int* need = c->d_need + l;
-  if (!g.brute) {
+  if (!g.brute && c->n <= kOneBlockAtoms && g.ncell <= kOneBlockCells) {
+    LAUNCH_ON(c, st, "nl_cells", k_cells, 1, kOneBlockThreads, S, g, need);
+  } else if (!g.brute) {
     LAUNCH_ON(c, st, "nl_cell_count", k_cell_count, nblk(c->n), kThreads, S, g, need);
     LAUNCH_ON(c, st, "nl_cell_scan", k_cell_scan, 1, 1024, g, need);
     LAUNCH_ON(c, st, "nl_cell_fill", k_cell_fill, nblk(c->n), kThreads, S, g, need);

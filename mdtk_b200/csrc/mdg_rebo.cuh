@@ -103,13 +103,14 @@ struct SinkT {
 };
 typedef SinkT<double> Sink;
 
-// s += a b.  In double each operation is rounded on its own, so that N^conj,
-// whose last bit the pi^rc cells' monomials magnify a million times, is the
-// same number in every kernel (and the reference's).
-template <class Real>
+// s += a b.  SPLIT, in double: each operation is rounded on its own, so that
+// N^conj, whose last bit the pi^rc cells' monomials magnify a million times, is
+// the same number in every split of the bond tasks (and the reference's).  The
+// special LJ pairs have one kernel each way and leave it to the compiler.
+template <bool SPLIT, class Real>
 MDG_HD void add_prod(Real& s, Real a, Real b)
 {
-  if constexpr (std::is_same<Real, double>::value) s = add_rn(s, mul_rn(a, b));
+  if constexpr (SPLIT && std::is_same<Real, double>::value) s = add_rn(s, mul_rn(a, b));
   else s += a * b;
 }
 
@@ -427,7 +428,7 @@ struct ReboT {
       if (k == o || type(k) != kC) continue;
       Real f = ld(&B.bu[q].w);
       Real N = Nk_excl(k, ld(&B.brv[q].w), f, c);
-      add_prod(sum, f, Sprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1])));
+      add_prod<RO>(sum, f, Sprime(N, ld(&P.Ntot[0]), ld(&P.Ntot[1])));
     }
     return sum;
   }
@@ -467,8 +468,8 @@ struct ReboT {
     s1 = nconj_sum(i, j);
     s2 = nconj_sum(j, i);
     Real N = 1.0;
-    add_prod(N, s1, s1);
-    add_prod(N, s2, s2);
+    add_prod<RO>(N, s1, s1);
+    add_prod<RO>(N, s2, s2);
     return N;
   }
   template <class S>
