@@ -3181,9 +3181,7 @@ int mdg_nl_pairs(mdg_ctx* c, int list_id, int32_t* pairs, int64_t cap, int64_t* 
 //   - the split: one task per directed bond, or one per bond (both route the
 //     same terms into the same records, equal to rounding);
 //   - with the LJ term, where the REBO tasks run: in order before the LJ
-//     chain with the grid at the kernel's resident capacity, or on the second
-//     stream concurrently with the LJ chain with 1, 2 or all resident blocks
-//     per SM (fewer blocks leave the SMs' registers to the LJ kernels).
+//     chain, or on the second stream concurrently with it.
 // The choice changes only the speed; results are bitwise the same for a
 // given split.
 // Time one force evaluation as the steps run it: captured into a CUDA graph
