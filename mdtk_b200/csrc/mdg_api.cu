@@ -137,6 +137,36 @@ __global__ void k_step_start(State S, StepDev P, int do_pos, NList L0, NList L1,
   if (threadIdx.x == 0) *done = 0u;
 }
 
+// Ascending order of v[0..n), distinct ints, by a whole warp: up to 128 by rank
+// (an LJ cell of diamond holds ~88 atoms), more by one lane's insertion sort.
+__device__ __forceinline__ void warp_sort(int* v, int n)
+{
+  const int lane = threadIdx.x & 31;
+  if (n <= 1) return;
+  if (n > 128) {
+    if (lane == 0) isort(v, n);
+    __syncwarp();
+    return;
+  }
+  int x[4], r[4] = {0, 0, 0, 0};
+#pragma unroll
+  for (int k = 0; k < 4; k++) x[k] = lane + 32 * k < n ? v[lane + 32 * k] : 0x7fffffff;
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    if (32 * k >= n) break;
+    for (int s = 0; s < 32; s++) {  // (the filler past n is larger than every entry)
+      const int y = __shfl_sync(0xffffffffu, x[k], s);
+#pragma unroll
+      for (int q = 0; q < 4; q++) r[q] += y < x[q];
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < 4; k++)
+    if (lane + 32 * k < n) v[r[k]] = x[k];
+  __syncwarp();
+}
+
 __global__ void k_cell_count(State S, Grid g, const int* need)
 {
   pdl_enter();
@@ -196,8 +226,9 @@ __global__ void k_cell_sort(Grid g, const int* need)
 // The four kernels above in one block, for systems of up to kOneBlockAtoms
 // atoms and kOneBlockCells cells.  A step launches them whether a rebuild is due
 // or not, and a kernel that returns at once still costs 2 us of the step's
-// chain; one block takes about CELLS_US us for the rebuild of 43,680 atoms, due
-// every ~30 steps, and beyond these sizes that outweighs the launches.
+// chain (1,728 diamond atoms: 53 us a step with them, 50 so).  One block takes
+// 14 us for the cells of those, 80 for a list of 16,128 ethane atoms and 200 for
+// one of 43,680; beyond these sizes that outweighs the launches.
 constexpr int kOneBlockAtoms = 65536, kOneBlockCells = 262144, kOneBlockThreads = 1024;
 __global__ void __launch_bounds__(kOneBlockThreads) k_cells(State S, Grid g, const int* need)
 {
@@ -238,15 +269,121 @@ __global__ void __launch_bounds__(kOneBlockThreads) k_cells(State S, Grid g, con
   }
   __threadfence();
   __syncthreads();
+  // ascending order inside each cell: a thread a cell while cells hold a few
+  // atoms (the REBO range), a warp a cell when they hold many (the LJ range)
+  if (S.n < 8 * g.ncell) {
+    for (int c = t; c < g.ncell; c += kOneBlockThreads) {
+      const int b = __ldcg(&g.cstart[c]), e = __ldcg(&g.cstart[c + 1]);
+      isort(g.catoms + b, e - b);
+    }
+  } else {
+    for (int c = wid; c < g.ncell; c += kOneBlockThreads / 32) {
+      const int b = __ldcg(&g.cstart[c]), e = __ldcg(&g.cstart[c + 1]);
+      warp_sort(g.catoms + b, e - b);
+    }
+  }
   for (int c = t; c < g.ncell; c += kOneBlockThreads) {
-    const int b = __ldcg(&g.cstart[c]), e = __ldcg(&g.cstart[c + 1]);
-    isort(g.catoms + b, e - b);
     g.ccount[c] = 0;
     g.ccursor[c] = 0;
   }
 }
 
-__global__ void k_nl_build(State S, Grid g, NList L, const int* need, unsigned int* status)
+// Verlet lists, a warp per atom over a resident grid: nl_build_atom's list (the
+// same cells in the same order, ascending when sorted), its lanes testing 32
+// candidates at a time (the LJ list of 43,680 ethane atoms, due every ~80 steps:
+// 690 us on a thread an atom, 370 so; the REBO list of 1,728 diamond atoms, due
+// on a first call: 90 and 23).
+__global__ void __launch_bounds__(kThreads) k_nl_build(State S, Grid g, NList L, const int* need,
+                                                       unsigned int* status)
+{
+  pdl_enter();
+  if (!*need) return;
+  const int lane = threadIdx.x & 31, nw = (gridDim.x * blockDim.x) >> 5;
+  const unsigned below = (1u << lane) - 1u;
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < S.n; i += nw) {  // whole warps
+    const double4 pi = S.pos[i];
+    const V3 xi = v3(pi.x, pi.y, pi.z);
+    const Box box = box_of(S, i);
+    int* out = L.list + (long)i * L.cap;
+    // FGeneral's handled pairs: REBO and AIREBO never see metal or ion atoms
+    const bool ich = pi.w < 1.5, none = L.pairs == 1 && !ich;
+    int cnt = 0;
+    // the candidates catoms[b..e) (or the atoms b..e themselves), in order
+    auto scan = [&](int b, int e, bool cells) {
+      for (int q0 = b; q0 < e; q0 += 32) {
+        const int q = q0 + lane;
+        bool in = false;
+        int j = -1;
+        if (q < e) {
+          j = cells ? g.catoms[q] : q;
+          if (j != i) {
+            const double4 pj = S.pos[j];
+            if (!(L.pairs && (L.pairs == 1 ? pj.w > 1.5 : (ich && pj.w < 1.5))))
+              in = norm2(depos(box, xi, v3(pj.x, pj.y, pj.z))) < L.range2;
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, in);
+        const int p = cnt + __popc(m & below);
+        if (in && p < L.cap) out[p] = j;
+        cnt += __popc(m);
+      }
+    };
+    if (none) {
+    } else if (g.brute && !S.sys) {
+      scan(0, S.n, false);
+    } else {
+      const GridView v = grid_view(g, S, i);
+      int c0[3], dlo[3], dhi[3];
+#pragma unroll
+      for (int ax = 0; ax < 3; ax++) {
+        c0[ax] = cell_coord(v, box, ax, ax == 0 ? pi.x : (ax == 1 ? pi.y : pi.z));
+        dlo[ax] = -1;
+        dhi[ax] = 1;
+        if (box.pbc[ax] && v.nc[ax] < 3) { dlo[ax] = 0; dhi[ax] = v.nc[ax] - 1; }
+      }
+      // a row of cells that crosses no border is one range of catoms
+      const bool row = c0[0] + dlo[0] >= 0 && c0[0] + dhi[0] < v.nc[0];
+      for (int dz = dlo[2]; dz <= dhi[2]; dz++) {
+        int cz = c0[2] + dz;
+        if (box.pbc[2]) cz = (cz + v.nc[2]) % v.nc[2];
+        else if (cz < 0 || cz >= v.nc[2]) continue;
+        for (int dy = dlo[1]; dy <= dhi[1]; dy++) {
+          int cy = c0[1] + dy;
+          if (box.pbc[1]) cy = (cy + v.nc[1]) % v.nc[1];
+          else if (cy < 0 || cy >= v.nc[1]) continue;
+          const int r0 = v.base + (cz * v.nc[1] + cy) * v.nc[0];
+          if (row) {
+            scan(g.cstart[r0 + c0[0] + dlo[0]], g.cstart[r0 + c0[0] + dhi[0] + 1], true);
+          } else {
+            for (int dx = dlo[0]; dx <= dhi[0]; dx++) {
+              int cx = c0[0] + dx;
+              if (box.pbc[0]) cx = (cx + v.nc[0]) % v.nc[0];
+              else if (cx < 0 || cx >= v.nc[0]) continue;
+              scan(g.cstart[r0 + cx], g.cstart[r0 + cx + 1], true);
+            }
+          }
+        }
+      }
+      if (L.sorted && cnt <= L.cap) {
+        __syncwarp();
+        warp_sort(out, cnt);
+      }
+    }
+    if (lane == 0) {
+      if (cnt > L.cap) atomicOr(status, ST_NL_OVERFLOW);
+      L.cnt[i] = min(cnt, L.cap);
+      L.pos0[i] = pi;
+    }
+  }
+}
+
+// The same, a thread per atom, once threads alone fill the GPU.  The REBO range:
+// cells hold about two atoms and leave most lanes of a warp without a candidate
+// (43,680 ethane atoms: 155 us on warps, 86 on threads; even at 16,128, 76 and
+// 81).  The longer ranges: 512,000 diamond atoms 6.40 ms on warps and 4.23 on
+// threads, 43,680 ethane atoms 370 us and 690.
+constexpr int kNlThreadAtomsRebo = 16384, kNlThreadAtoms = 131072;
+__global__ void k_nl_build_thread(State S, Grid g, NList L, const int* need, unsigned int* status)
 {
   pdl_enter();
   if (!*need) return;
@@ -1857,6 +1994,7 @@ struct mdg_ctx {
 
   unsigned int* d_status = nullptr;
   int special_blocks = 0;
+  int nl_blocks = 0;          // resident blocks of the list build (grid-stride over atoms)
   int cij_blocks = 0;         // resident blocks of the connectivity kernel (grid-stride over atoms)
   int* cij_scratch = nullptr; // its candidates, a row per resident group
   int warp_blocks = 0;        // resident blocks of the warp-per-atom LJ list kernels (grid-stride over atoms)
@@ -2297,8 +2435,11 @@ int rebuild_list(mdg_ctx* c, int l, cudaStream_t st)
     LAUNCH_ON(c, st, "nl_cell_fill", k_cell_fill, nblk(c->n), kThreads, S, g, need);
     LAUNCH_ON(c, st, "nl_cell_sort", k_cell_sort, nblk(g.ncell), kThreads, g, need);
   }
-  LAUNCH_ON(c, st, l == 0 ? "nl_build_rebo" : (l == 1 ? "nl_build_lj" : "nl_build_metal"), k_nl_build, nblk(c->n),
-            kThreads, S, g, L, need, c->d_status);
+  const char* name = l == 0 ? "nl_build_rebo" : (l == 1 ? "nl_build_lj" : "nl_build_metal");
+  if (c->n > (l == 0 ? kNlThreadAtomsRebo : kNlThreadAtoms))
+    LAUNCH_ON(c, st, name, k_nl_build_thread, nblk(c->n), kThreads, S, g, L, need, c->d_status);
+  else
+    LAUNCH_ON(c, st, name, k_nl_build, std::min(nblk(c->n * 32), c->nl_blocks), kThreads, S, g, L, need, c->d_status);
   if (l == 1)
     LAUNCH_ON(c, st, "nl_build_lj_near", k_lj_near, std::min(nblk(c->n * 32), c->warp_blocks), kThreads, c->ljp, S,
               L, c->ljt, c->d_need, c->d_status);
@@ -2874,6 +3015,13 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     int rc = nsys > 1 ? setup_grid_batch(c, l, hpos) : setup_grid(c, l, hpos);
     if (rc) return rc;
   }
+  {
+    int dev = 0, sms = 148, per = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_nl_build, kThreads, 0);
+    c->nl_blocks = sms * (per > 0 ? per : 1);
+  }
   int one[4] = {1, 1, 1, 1};
   CK(cudaMemcpy(c->d_force, one, sizeof(one), cudaMemcpyHostToDevice));
   c->d_part = dalloc<double>(2 * 4 * kDispParts);
@@ -3239,14 +3387,13 @@ static int autotune(mdg_ctx* c)
   if (c->prm.task_mode != 0 && !lj) return MDG_OK;
   const int mode0 = c->prm.task_mode ? c->prm.task_mode - 1 : 0;
   const int mode1 = c->prm.task_mode ? c->prm.task_mode : 3;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // Beside the LJ chain the REBO tasks get all resident blocks: at the ideal
+  // bond lengths of a fresh system two blocks an SM can read 1.5% faster, but
+  // once its bonds stretch into the cutoffs' windows the tasks grow (43,680
+  // ethane atoms after 40 fs, one task per bond: 264 us a step on 444 blocks, 275 on 296,
+  // 322 on 148).
   struct Cfg { bool overlap; int grid; };
   std::vector<Cfg> cfgs = {{false, c->rebo_task_blocks}};
-  if (lj)
-    for (int per : {1, 2})
-      if (sms * per < c->rebo_task_blocks) cfgs.push_back({true, sms * per});
   if (lj) cfgs.push_back({true, c->rebo_task_blocks});
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
