@@ -24,7 +24,7 @@ RANGE = (1.44 * 2.0, 1.44 * 5.5)
 
 def _pairs(pos, s, r):
     span = np.where(s["pbc"] != 0, s["box"], 1e4)
-    x = np.where(s["pbc"] != 0, np.mod(pos, s["box"]), pos - pos.min(axis=0) + 1.0)
+    x = np.where(s["pbc"] != 0, np.mod(pos, span), pos - pos.min(axis=0) + 1.0)
     p = cKDTree(x, boxsize=span).query_pairs(r, output_type="ndarray")
     p.sort(axis=1)
     return p[np.lexsort((p[:, 1], p[:, 0]))].astype(np.int32)
