@@ -1635,6 +1635,7 @@ int mdg_set_images(mdg_ctx* c, const int32_t* image)
   if (!image) return fail(MDG_ERR_ARG, "null argument");
   std::vector<int4> h(c->n);
   for (int i = 0; i < c->n; i++) h[i] = make_int4(image[3 * i], image[3 * i + 1], image[3 * i + 2], 0);
+  CK(cudaStreamSynchronize(c->stream));  // a state set before this counts its periods first
   CK(cudaMemcpy(c->image, h.data(), c->n * sizeof(int4), cudaMemcpyHostToDevice));
   return MDG_OK;
 }
