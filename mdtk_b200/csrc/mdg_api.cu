@@ -1031,7 +1031,7 @@ __global__ void __launch_bounds__(kCijThreads) k_cij(BondList B, CijTable T, int
     const bool live = a < B.n;
     const int nb1 = live ? B.nb[a] : 0;
     const int q1 = a * B.mb;
-    bool wide = nb1 > kCijGroup || B.mb > 32;
+    bool wide = nb1 > kCijGroup;
     // lane s holds the s-th partner, its bond count and weight
     const bool has = gl < nb1 && !wide;
     const int k1 = has ? B.bj[q1 + gl] : 0;
@@ -1162,6 +1162,21 @@ __global__ void __launch_bounds__(kCijThreads) k_cij(BondList B, CijTable T, int
     }
     __syncwarp();  // this atom's candidates are read before the next one's are laid down
   }
+}
+
+// The one-thread build for every atom: contexts whose bond capacity is beyond
+// the codes' five bits a slot (32).  A kernel of its own, since on one lane of
+// each of k_cij's groups seven eighths of the lanes wait: 575 us so on 64,000
+// diamond atoms with a capacity of 40, 231 here; 131 by groups (capacity 16).
+__global__ void __launch_bounds__(kCijThreads) k_cij_thread(BondList B, CijTable T, unsigned long long* spc_ctr,
+                                                            unsigned char* mflag, unsigned int* status)
+{
+  pdl_enter();
+  const int a = blockIdx.x * blockDim.x + threadIdx.x;
+  if (a == 0 && spc_ctr) spc_ctr[0] = spc_ctr[kCtrStride] = spc_ctr[2 * kCtrStride] = 0ull;
+  if (a >= B.n) return;
+  mflag[a] = 0;
+  cij_build_atom<kCijLocal>(B, T, a, status);
 }
 
 // The LJ list's near sublist: the entries within R2 + kLjNearSkin of the
@@ -2583,8 +2598,12 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
   if (!tasks && (pot & MDG_POT_BRENNER))
     LAUNCH(c, "brenner", k_brenner, nblk(c->n), kThreads, c->d_bp, c->d_btables, B, c->fo, c->d_status);
   if (lj) {
-    LAUNCH(c, "cij_table", k_cij, std::min(nblk(c->n, kCijAtoms), c->cij_blocks), kCijThreads, B, c->cij,
-           c->cij_scratch, c->spc.ctr, c->spc.mflag, c->d_status);
+    if (c->mb > 32)
+      LAUNCH(c, "cij_table", k_cij_thread, nblk(c->n, kCijThreads), kCijThreads, B, c->cij, c->spc.ctr, c->spc.mflag,
+             c->d_status);
+    else
+      LAUNCH(c, "cij_table", k_cij, std::min(nblk(c->n, kCijAtoms), c->cij_blocks), kCijThreads, B, c->cij,
+             c->cij_scratch, c->spc.ctr, c->spc.mflag, c->d_status);
     if (ovl) CK(cudaStreamWaitEvent(c->stream, c->ev_join2, 0));
     const int pairs = (c->bt.ctr && c->bt.pairs) ? 1 : 0;
     const int lgrid = nblk(c->n * kLjGroup, kLjThreads);
