@@ -2174,6 +2174,14 @@ void io_free(mdg_ctx* c);
 void snap_free(mdg_ctx* c);
 int snap_capture(mdg_ctx* c);
 
+void free_bond_tasks(mdg_ctx* c)
+{
+  void* bq[] = {c->bt.q, c->bt.ctr, c->bt.rbase, c->bt.nrec, c->bt.rec};
+  for (void* p : bq)
+    if (p) cudaFree(p);
+  std::memset(&c->bt, 0, sizeof(c->bt));
+}
+
 void free_system(mdg_ctx* c)
 {
   io_release(c);
@@ -2240,10 +2248,7 @@ void free_system(mdg_ctx* c)
   c->h_first.clear();
   c->h_boxes.clear();
   c->h_sys.clear();
-  void* bq[] = {c->bt.q, c->bt.ctr, c->bt.rbase, c->bt.nrec, c->bt.rec};
-  for (void* p : bq)
-    if (p) cudaFree(p);
-  std::memset(&c->bt, 0, sizeof(c->bt));
+  free_bond_tasks(c);
   if (c->stage_busy) cudaEventSynchronize(c->ev_stage);
   c->stage_busy = false;
   if (c->h_stage) cudaFreeHost(c->h_stage);
@@ -3086,14 +3091,20 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     return fail(MDG_ERR_CUDA, "cudaMalloc (bonds)");
   CK(cudaMemset(c->fo.glj, 0, n * sizeof(double4)));
   CK(cudaMemset(c->fo.e_lj, 0, n * sizeof(double)));
-  // Brenner's records are sized for atoms with every bond slot in use (its
-  // per-atom kernel has no such limit); beyond kBrennerRecBytes that kernel is
-  // taken instead.
+  // Brenner's records are sized for atoms with every bond slot in use.  Its
+  // per-atom kernel needs none: it is taken beyond kBrennerRecBytes, when the
+  // records would leave less memory free than they take, and when they cannot
+  // be had after all.
   const bool brenner = c->prm.potentials & MDG_POT_BRENNER;
   const int tors1 = (c->prm.potentials & MDG_POT_ETORS) ? 1 : 0;
   const double brenner_rec = (double)n * mb * (1 + tors1) * bond_rec_size(mb);
-  if (brenner ? brenner_rec * sizeof(double) <= kBrennerRecBytes
-              : (c->prm.potentials & (MDG_POT_REBO | MDG_POT_ETORS)) != 0) {
+  bool tasks = brenner || tors1 || (c->prm.potentials & MDG_POT_REBO);
+  if (brenner) {
+    size_t mem_free = 0, mem_total = 0;
+    CK(cudaMemGetInfo(&mem_free, &mem_total));
+    tasks = brenner_rec * sizeof(double) <= std::min(kBrennerRecBytes, 0.5 * (double)mem_free);
+  }
+  if (tasks) {
     BondTasks& K = c->bt;
     K.cap = n * mb;
     K.pairs = brenner ? 2 : (c->prm.task_mode >= 2 ? c->prm.task_mode - 1 : 0);
@@ -3104,8 +3115,14 @@ static int set_systems(mdg_ctx* c, int nsys, const int64_t* first, const int32_t
     K.rbase = dalloc<long>(n);
     K.nrec = dalloc<int>(n);
     K.rec = dalloc<double>((size_t)K.rec_cap);
-    if (!K.q || !K.ctr || !K.rbase || !K.nrec || !K.rec) return fail(MDG_ERR_CUDA, "cudaMalloc (bond tasks)");
-    CK(cudaMemset(K.ctr, 0, 3 * kTaskCtr * sizeof(unsigned long long)));
+    if (!K.q || !K.ctr || !K.rbase || !K.nrec || !K.rec) {
+      if (!brenner) return fail(MDG_ERR_CUDA, "cudaMalloc (bond tasks)");
+      free_bond_tasks(c);
+      cudaGetLastError();  // (the failed allocation's)
+    }
+  }
+  if (c->bt.ctr) {
+    CK(cudaMemset(c->bt.ctr, 0, 3 * kTaskCtr * sizeof(unsigned long long)));
     int dev = 0, sms = 148, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
