@@ -3854,11 +3854,16 @@ int mdg_get_state(mdg_ctx* c, double* pos, double* vel, int32_t* image)
     if (image) std::memcpy(image, c->h_stage + 6 * (size_t)n, 3 * (size_t)n * sizeof(int32_t));
     return MDG_OK;
   }
+  // straight into the caller's arrays, once the status is known: after an
+  // error they stay as they were
+  int rc = read_status(c);
+  if (rc) return rc;
   if (pos) CK(cudaMemcpyAsync(pos, io, bytes, cudaMemcpyDeviceToHost, c->stream));
   if (vel) CK(cudaMemcpyAsync(vel, io + 3 * (size_t)n, bytes, cudaMemcpyDeviceToHost, c->stream));
   if (image)
     CK(cudaMemcpyAsync(image, io + 6 * (size_t)n, 3 * (size_t)n * sizeof(int32_t), cudaMemcpyDeviceToHost, c->stream));
-  return read_status(c);
+  CK(cudaStreamSynchronize(c->stream));
+  return MDG_OK;
 }
 
 int64_t mdg_launch_count(mdg_ctx* c) { return c ? c->launches : 0; }
