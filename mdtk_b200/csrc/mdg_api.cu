@@ -3381,6 +3381,9 @@ static int time_eval_graph(mdg_ctx* c, cudaEvent_t e0, cudaEvent_t e1, float* be
   std::memset(&still, 0, sizeof(still));
   still.nlc0 = c->nl[0].cnt;
   const bool step = !c->acc_valid && !c->snap;
+  // stale accelerations may not be finite (a diverged run before the state was
+  // set again), and 0 times those is not 0
+  if (step) CK(cudaMemsetAsync(c->acc, 0, c->n * sizeof(double4), c->stream));
   cudaGraph_t g = nullptr;
   cudaGraphExec_t ge = nullptr;
   const int64_t l0 = c->launches;
