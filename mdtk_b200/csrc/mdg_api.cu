@@ -2866,8 +2866,12 @@ int mdg_set_stream(mdg_ctx* c, void* stream)
 {
   if (!c) return fail(MDG_ERR_ARG, "null context");
   cudaStream_t next = stream ? (cudaStream_t)stream : c->own_stream;
-  // a state on its way to the device is not left behind on the old stream
-  if (next != c->stream && c->stage_busy) CK(cudaStreamSynchronize(c->stream));
+  // a state on its way to the device is not left behind on the old stream,
+  // which its owner may have destroyed by now: the event is the context's own
+  if (next != c->stream) {
+    int rc = stage_wait(c);
+    if (rc) return rc;
+  }
   c->stream = next;
   return MDG_OK;
 }

@@ -2,6 +2,8 @@
 box with their image counts, calls that follow mdg_set_state directly, and the
 caller's arrays when the device reports an error.  States up to 4,096 atoms
 pass through pinned memory in one copy, larger ones do not."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -88,3 +90,20 @@ def test_arrays_stay_when_the_device_reports_an_error(cells):
     assert M.lib().mdg_get_state(ctx.h, M._dp(out[0]), None, M._ip(out[2])) == 0  # the error is reported once
     assert np.all(np.isfinite(out[0])) and not np.array_equal(out[0], mark[0])
     assert np.array_equal(out[1], mark[1])
+
+
+def test_stream_destroyed_before_the_next_is_set():
+    """A caller may destroy a stream as soon as its own calls on it are done;
+    the state on its way there is waited for through the context's own event."""
+    cu = ctypes.CDLL("libcuda.so.1")
+    s = B.diamond(4, temp_k=300.0, disp_sigma=0.05, seed=208)
+    ctx = _load(s)
+    x, w, _ = _moved(s, 209)
+    for _ in range(3):
+        stream = ctypes.c_void_p()
+        assert cu.cuStreamCreate(ctypes.byref(stream), 1) == 0  # CU_STREAM_NON_BLOCKING
+        ctx.set_stream(stream.value)
+        ctx.set_state(x)
+        assert cu.cuStreamDestroy_v2(stream) == 0
+        ctx.set_stream(0)
+        assert np.array_equal(ctx.get_state()[0], w)
