@@ -47,7 +47,7 @@ struct AdjWs {
   dual4 *brv = nullptr, *bu = nullptr, *bd = nullptr, *nco = nullptr;
   dual *A = nullptr, *W = nullptr, *er = nullptr, *et = nullptr, *el = nullptr, *dp = nullptr;
   dual4 *gown = nullptr, *glj = nullptr, *g = nullptr;
-  dual* brec = nullptr;               // bond-slot records (adj_rec_size)
+  dual* brec = nullptr;               // bond-slot records (adj_rec_size); null: they lie in trec
   long brcap = 0;                     // record doubles of the FP64 path they were sized by
   dual* cw = nullptr;                 // connectivity weights
   dual *trec = nullptr, *tmidc = nullptr, *tdp = nullptr;  // special-pair task records
@@ -438,8 +438,13 @@ int adj_ensure(mdg_ctx* c)
             adj_realloc(w->lx, (size_t)n) && adj_realloc(w->lv, (size_t)n) && adj_realloc(w->la, (size_t)n) &&
             adj_realloc(w->theta, kNParam) && adj_realloc(w->dpar, 2 * kNParam) &&
             adj_realloc(w->fin_pos, (size_t)n) && adj_realloc(w->fin_vel, (size_t)n) &&
-            adj_realloc(w->fin_acc, (size_t)n) && adj_realloc(w->fin_img, (size_t)n) &&
-            adj_realloc(w->brec, 2 * (size_t)c->bt.rec_cap);
+            adj_realloc(w->fin_acc, (size_t)n) && adj_realloc(w->fin_img, (size_t)n);
+  // the bond-slot records are summed before the special-pair tasks write
+  // theirs, and take the same memory where it is large enough (at the default
+  // capacities it is)
+  if (w->brec) cudaFree(w->brec);
+  w->brec = nullptr;
+  if (2 * c->bt.rec_cap > rcap) ok = ok && adj_realloc(w->brec, 2 * (size_t)c->bt.rec_cap);
   if (!ok) return fail(MDG_ERR_CUDA, "cudaMalloc (adjoint buffers)");
   // the glj of a context without the LJ term stays zero; no task holds a
   // middle bond before the first pass
@@ -493,9 +498,10 @@ int adj_dual_pass(mdg_ctx* c, int transpose = 1)
   O.e_lj = w->el;
   O.dp = w->dp;
   O.jt = transpose;
+  dual* brec = w->brec ? w->brec : w->trec;
   LAUNCH(c, "adj_rebo_tors", k_adj_rebo, nblk(n * kAdjLanes, 64), 64, c->d_rp, c->d_tables, DB, c->tp, rebo ? 1 : 0,
-         tors ? 1 : 0, transpose, c->bt.rbase, w->brec, c->d_status);
-  LAUNCH(c, "adj_bond_reduce", k_adj_bond_reduce, nblk(n * kReduceLanes), kThreads, DB, c->bt.rbase, w->brec, O);
+         tors ? 1 : 0, transpose, c->bt.rbase, brec, c->d_status);
+  LAUNCH(c, "adj_bond_reduce", k_adj_bond_reduce, nblk(n * kReduceLanes), kThreads, DB, c->bt.rbase, brec, O);
   SpecialTasksT<dual> Tk;
   std::memset(&Tk, 0, sizeof(Tk));
   if (lj) {
