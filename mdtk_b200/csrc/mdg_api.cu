@@ -223,66 +223,85 @@ __global__ void k_cell_sort(Grid g, const int* need)
   g.ccursor[c] = 0;
 }
 
-// The four kernels above in one block, for systems of up to kOneBlockAtoms
-// atoms and kOneBlockCells cells.  A step launches them whether a rebuild is due
-// or not, and a kernel that returns at once still costs 2 us of the step's
-// chain (1,728 diamond atoms: 53 us a step with them, 50 so).  One block takes
-// 14 us for the cells of those, 80 for a list of 16,128 ethane atoms and 200 for
-// one of 43,680; beyond these sizes that outweighs the launches.
-constexpr int kOneBlockAtoms = 65536, kOneBlockCells = 262144, kOneBlockThreads = 1024;
-__global__ void __launch_bounds__(kOneBlockThreads) k_cells(State S, Grid g, const int* need)
+// The four kernels above in one, on a cluster of eight blocks (its barrier
+// between the phases), for systems of up to kCellsAtoms atoms and kCellsCells
+// cells.  A step launches them whether a rebuild is due or not, and a kernel
+// that returns at once still costs about 1 us of the step's chain.  A rebuild is
+// bound by the latency of the position loads and atomics of the few atoms a
+// thread takes in turn, and by the scan, which one block makes.  One block for
+// all of it rebuilt on one SM and lost more than it gained where rebuilds are
+// frequent (a thin skin, a fast projectile, frames that lie far apart).  Us a
+// step, four kernels / one block / the cluster, without a rebuild and with one
+// at every step:
+//   diamond 4,096 (REBO)    63.8 /  61.7 /  60.8     96 /   105 /  97
+//   diamond 21,952          91.3 /  87.8 /  87.9    158 /   232 / 170
+//   diamond 64,000         236.8 / 233.1 / 234.0    336 /   553 / 375
+//   ethane 4,368 (AIREBO)  103.0 / 100.1 /  99.7    186 /   172 / 149
+//   ethane 17,472          152.8 / 149.4 / 149.6    351 /   381 / 300
+//   ethane 43,680          265.1 / 260.0 / 260.6    566 /   787 / 572
+//   Cu slab 19,233         167.6 / 161.6 / 159.9    327 /   520 / 301
+//   gas of 4,000, 27,000 cells  74.7 / 71.9 / 72.0  112 /   135 / 122
+//   gas of 4,000, 216,000       75.9 / 73.7 / 72.9  300 /   399 / 352
+// Beyond the limits a rebuild at every tenth step would cost what the others save.
+constexpr int kCellsAtoms = 49152, kCellsCells = 32768, kCellsThreads = 1024, kCellsBlocks = 8;
+__global__ void __cluster_dims__(kCellsBlocks, 1, 1) __launch_bounds__(kCellsThreads)
+    k_cells(State S, Grid g, const int* need)
 {
   pdl_enter();
   if (!*need) return;
-  __shared__ int wsum[kOneBlockThreads / 32];
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
-  for (int i = t; i < S.n; i += kOneBlockThreads) atomicAdd(&g.ccount[cell_of(g, S, i)], 1);
+  __shared__ int wsum[kCellsThreads / 32];
+  const auto cluster = cooperative_groups::this_cluster();
+  constexpr int all = kCellsThreads * kCellsBlocks;
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, rank = (int)cluster.block_rank(), ct = rank * kCellsThreads + t;
+  for (int i = ct; i < S.n; i += all) atomicAdd(&g.ccount[cell_of(g, S, i)], 1);
   __threadfence();
-  __syncthreads();
-  // exclusive scan of the counts, a tile of one cell a thread at a time
-  int carry = 0;  // the same in every thread
-  for (int b = 0; b < g.ncell; b += kOneBlockThreads) {
-    const int v = b + t < g.ncell ? __ldcg(&g.ccount[b + t]) : 0;
-    int x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += y;
+  cluster.sync();
+  if (rank == 0) {
+    // exclusive scan of the counts, a tile of one cell a thread at a time
+    int carry = 0;  // the same in every thread
+    for (int b = 0; b < g.ncell; b += kCellsThreads) {
+      const int v = b + t < g.ncell ? __ldcg(&g.ccount[b + t]) : 0;
+      int x = v;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) wsum[wid] = x;
+      __syncthreads();
+      int before = 0, total = 0;
+      for (int w = 0; w < kCellsThreads / 32; w++) {
+        const int s = wsum[w];
+        if (w < wid) before += s;
+        total += s;
+      }
+      if (b + t < g.ncell) g.cstart[b + t] = carry + before + x - v;
+      carry += total;
+      __syncthreads();
     }
-    if (lane == 31) wsum[wid] = x;
-    __syncthreads();
-    int before = 0, total = 0;
-    for (int w = 0; w < kOneBlockThreads / 32; w++) {
-      const int s = wsum[w];
-      if (w < wid) before += s;
-      total += s;
-    }
-    if (b + t < g.ncell) g.cstart[b + t] = carry + before + x - v;
-    carry += total;
-    __syncthreads();
+    if (t == 0) g.cstart[g.ncell] = carry;
   }
-  if (t == 0) g.cstart[g.ncell] = carry;
   __threadfence();
-  __syncthreads();
-  for (int i = t; i < S.n; i += kOneBlockThreads) {
+  cluster.sync();
+  for (int i = ct; i < S.n; i += all) {
     const int c = cell_of(g, S, i);
     g.catoms[__ldcg(&g.cstart[c]) + atomicAdd(&g.ccursor[c], 1)] = i;
   }
   __threadfence();
-  __syncthreads();
+  cluster.sync();
   // ascending order inside each cell: a thread a cell while cells hold a few
   // atoms (the REBO range), a warp a cell when they hold many (the LJ range)
   if (S.n < 8 * g.ncell) {
-    for (int c = t; c < g.ncell; c += kOneBlockThreads) {
+    for (int c = ct; c < g.ncell; c += all) {
       const int b = __ldcg(&g.cstart[c]), e = __ldcg(&g.cstart[c + 1]);
       isort(g.catoms + b, e - b);
     }
   } else {
-    for (int c = wid; c < g.ncell; c += kOneBlockThreads / 32) {
+    for (int c = ct >> 5; c < g.ncell; c += all / 32) {
       const int b = __ldcg(&g.cstart[c]), e = __ldcg(&g.cstart[c + 1]);
       warp_sort(g.catoms + b, e - b);
     }
   }
-  for (int c = t; c < g.ncell; c += kOneBlockThreads) {
+  for (int c = ct; c < g.ncell; c += all) {
     g.ccount[c] = 0;
     g.ccursor[c] = 0;
   }
@@ -2447,8 +2466,8 @@ int rebuild_list(mdg_ctx* c, int l, cudaStream_t st)
   NList& L = c->nl[l];
   Grid& g = c->grid[l];
   int* need = c->d_need + l;
-  if (!g.brute && c->n <= kOneBlockAtoms && g.ncell <= kOneBlockCells) {
-    LAUNCH_ON(c, st, "nl_cells", k_cells, 1, kOneBlockThreads, S, g, need);
+  if (!g.brute && c->n <= kCellsAtoms && g.ncell <= kCellsCells) {
+    LAUNCH_ON(c, st, "nl_cells", k_cells, kCellsBlocks, kCellsThreads, S, g, need);
   } else if (!g.brute) {
     LAUNCH_ON(c, st, "nl_cell_count", k_cell_count, nblk(c->n), kThreads, S, g, need);
     LAUNCH_ON(c, st, "nl_cell_scan", k_cell_scan, 1, 1024, g, need);

@@ -105,3 +105,20 @@ def test_tables_that_do_not_fit_are_reported(name):
         else:
             a, b = _force(s, cap_cij=24, **kw), _force(s, **kw)
             assert a[0] == b[0] and np.array_equal(a[2], b[2])
+
+
+@pytest.mark.parametrize("edge", [40.0, 90.0, 100.0])  # 2,197, 29,791 and 39,304 cells: the cluster, the cluster, four kernels
+def test_lists_of_a_gas_equal_a_kd_tree(edge):
+    m = B.c2h6_example()
+    place = (np.stack(np.meshgrid(*3 * [np.arange(3)], indexing="ij"), -1).reshape(-1, 1, 3) + 0.5) * edge / 3
+    pos = (place + m["pos"] - m["pos"].mean(axis=0)).reshape(-1, 3)
+    pos += np.random.default_rng(234).normal(scale=0.02, size=pos.shape)
+    ctx = M.Context(potentials=M.POT_REBO)
+    ctx.set_system(np.tile(m["z"], 27), pos, None, 3 * [edge])
+    for shift in (0.0, 0.37 * edge):  # the second time through the borders
+        x = np.mod(pos + shift, edge)
+        ctx.set_state(x)
+        want = cKDTree(x, boxsize=edge).query_pairs(1.44 * 2.0, output_type="ndarray")
+        want.sort(axis=1)
+        # (no pair lies within 1e-9 of the range)
+        assert np.array_equal(ctx.nl_pairs(0), want[np.lexsort((want[:, 1], want[:, 0]))])
