@@ -396,12 +396,13 @@ __global__ void __launch_bounds__(kThreads) k_nl_build(State S, Grid g, NList L,
   }
 }
 
-// The same, a thread per atom, once threads alone fill the GPU.  The REBO range:
-// cells hold about two atoms and leave most lanes of a warp without a candidate
-// (43,680 ethane atoms: 155 us on warps, 86 on threads; even at 16,128, 76 and
-// 81).  The longer ranges: 512,000 diamond atoms 6.40 ms on warps and 4.23 on
-// threads, 43,680 ethane atoms 370 us and 690.
-constexpr int kNlThreadAtomsRebo = 16384, kNlThreadAtoms = 131072;
+// The same, a thread per atom, once threads alone fill the GPU.  Us a build on
+// warps / on threads.  The REBO range, where cells hold about two atoms and
+// leave most lanes of a warp without a candidate: 17,472 ethane atoms 85 / 82,
+// 43,680 154 / 90; diamond 21,952 89 / 101, 46,656 160 / 128.  The longer
+// ranges: ethane 43,680 370 / 676, 87,360 709 / 707, 131,040 1,011 / 796;
+// diamond 64,000 791 / 1,098, 85,184 1,343 / 1,514, 140,608 2,062 / 1,611.
+constexpr int kNlThreadAtomsRebo = 16384, kNlThreadAtoms = 90000;
 __global__ void k_nl_build_thread(State S, Grid g, NList L, const int* need, unsigned int* status)
 {
   pdl_enter();
@@ -410,13 +411,15 @@ __global__ void k_nl_build_thread(State S, Grid g, NList L, const int* need, uns
   if (i < S.n) nl_build_atom(S, g, L, i, status);
 }
 
-// Lanes per atom of the bond list and the reverse slots: as long as eight times
-// the atoms fit the GPU's resident threads, an atom's list entries are spread
-// over eight lanes; beyond, over two (512,000 diamond atoms: bonds 240 and
-// reverse slots 72 us on eight lanes, 168 and 46 on two; a thread an atom took
-// 164 and 62).
+// Lanes per atom of the bond list and the reverse slots: eight spread an atom's
+// list entries while the system leaves lanes idle, two give fewer idle lanes
+// once it does not.  Us a step of REBO with two / with eight:
+//   diamond  8,000 71.7 / 63.8   21,952 89.0 / 88.3   32,768 133.5 / 134.5   262,144 763 / 783
+//   ethane   8,736 68.6 / 64.6   17,472 72.4 / 69.7   43,680  99.4 / 101.2   262,080 418 / 462
+// (a thread an atom took 164 us for the bonds of 512,000 diamond atoms and 62
+// for their reverse slots; two lanes take 168 and 46).
 constexpr int kBondLanes = 8, kBondLanesLarge = 2;
-constexpr int kBondLanesAtoms = 65536;
+constexpr int kBondLanesAtoms = 24576;
 
 // The bond list, LANES lanes per atom.  Bound by the latency of the position
 // gathers: a thread an atom walked its ~16 list entries in sequence (1,728
