@@ -240,7 +240,7 @@ __global__ void k_adj_lj_plain(LJParams P, CijTableT<dual> T, State S, int lcap,
   const int nf = live ? far_cnt[a] : 0;
   const int* row = inr + (long)a * lcap;
   const unsigned long long amask = T.mask[a];
-  for (int s = gl; s < nf; s += kLjGroup) lj_plain_pair<dual>(P, T, S, a, row[s], xa, ta, amask, sk, e, tan, true);
+  for (int s = gl; s < nf; s += kLjGroup) lj_plain_pair<dual>(P, T, S, a, row[s], xa, ta, amask, sk, e, tan);
   auto sum = [](dual x) {
     for (int o = kLjGroup / 2; o > 0; o >>= 1)
       x += dual(__shfl_xor_sync(0xffffffffu, x.v, o), __shfl_xor_sync(0xffffffffu, x.d, o));
@@ -497,7 +497,6 @@ int adj_dual_pass(mdg_ctx* c, int transpose = 1)
   O.e_tors = w->et;
   O.e_lj = w->el;
   O.dp = w->dp;
-  O.jt = transpose;
   dual* brec = w->brec ? w->brec : w->trec;
   LAUNCH(c, "adj_rebo_tors", k_adj_rebo, nblk(n * kAdjLanes, 64), 64, c->d_rp, c->d_tables, DB, c->tp, rebo ? 1 : 0,
          tors ? 1 : 0, transpose, c->bt.rbase, brec, c->d_status);

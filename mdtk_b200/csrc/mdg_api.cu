@@ -2015,7 +2015,6 @@ struct mdg_ctx {
   SpecialTasks spc;
   BondTasks bt;
   int rebo_task_blocks = 0;   // resident capacity of the REBO task kernel (blocks)
-  int rebo_grid = 0;          // blocks it is launched with (the autotuner's choice; 0 = capacity)
   // REBO tasks on a second stream, concurrent with the LJ chain (which does
   // not read their records until the reduction): fork/join by events, also
   // inside a captured step
@@ -2266,7 +2265,6 @@ void free_system(mdg_ctx* c)
   c->nsys = 1;
   c->tuned = false;
   c->overlap = false;
-  c->rebo_grid = 0;
   c->h_first.clear();
   c->h_boxes.clear();
   c->h_sys.clear();
@@ -2585,7 +2583,7 @@ int evaluate(mdg_ctx* c, const StepDev* step = nullptr)
            c->d_tables, B, c->tp, tors ? 1 : 0, c->bt, c->d_status);
   } else if (tasks) {
     const int ir = rebo ? 1 : 0, it = tors ? 1 : 0;
-    const int grid = c->rebo_grid > 0 ? c->rebo_grid : c->rebo_task_blocks;
+    const int grid = c->rebo_task_blocks;
     if (f32p && c->bt.pairs == 2) {
       auto kern = k_rebo_split_task<f32, ReboTables32>;
       LAUNCH_ON(c, rs, "rebo_tors", kern, grid, kThreads, c->d_rp, c->d_tables32, B, c->tp, ir, it, c->bt,
@@ -3385,22 +3383,24 @@ int mdg_nl_pairs(mdg_ctx* c, int list_id, int32_t* pairs, int64_t cap, int64_t* 
   return MDG_OK;
 }
 
-// The autotuner: with task_mode 0, on the first run of a system, times one
-// force evaluation (after one untimed evaluation; best of three) in each
-// configuration of the REBO work and keeps the fastest:
-//   - the split: one task per directed bond, or one per bond (both route the
-//     same terms into the same records, equal to rounding);
+// The autotuner: with task_mode 0, on the first run of a system, times each
+// configuration of the REBO work (after one untimed evaluation) and keeps the
+// fastest:
+//   - the split: one task per directed bond, one per bond, or bond ends on
+//     pairs of lanes (all route the same terms into the same records, equal to
+//     rounding);
 //   - with the LJ term, where the REBO tasks run: in order before the LJ
 //     chain, or on the second stream concurrently with it.
 // The choice changes only the speed; results are bitwise the same for a
 // given split.
-// Time one force evaluation as the steps run it: captured into a CUDA graph
-// (stream overlap and dependent launches included) and replayed four times
-// back to back per sample; the best of three samples, per evaluation.  Where
+// The timing of one configuration, as the steps run it: captured into a CUDA
+// graph (stream overlap and dependent launches included) and replayed four
+// times back to back per sample; the best of three samples, per replay.  Where
 // the accelerations are yet to be set (init_first_step follows), it is a whole
-// step of dt 0, which leaves the positions and velocities as they are: two
-// configurations whose bare evaluations differ by 0.1% took 273 and 286 us a
-// step on 43,680 ethane atoms.
+// step of dt 0, which leaves the positions and velocities as they are; where
+// they are set already, a bare force evaluation.  (Two configurations whose
+// bare evaluations differ by 0.1% took 273 and 286 us a step on 43,680 ethane
+// atoms.)
 static int time_eval_graph(mdg_ctx* c, cudaEvent_t e0, cudaEvent_t e1, float* best)
 {
   StepDev still;
@@ -3457,21 +3457,17 @@ static int autotune(mdg_ctx* c)
   // once its bonds stretch into the cutoffs' windows the tasks grow (43,680
   // ethane atoms after 40 fs, one task per bond: 264 us a step on 444 blocks, 275 on 296,
   // 322 on 148).
-  struct Cfg { bool overlap; int grid; };
-  std::vector<Cfg> cfgs = {{false, c->rebo_task_blocks}};
-  if (lj) cfgs.push_back({true, c->rebo_task_blocks});
   cudaEvent_t e0, e1;
   CK(cudaEventCreate(&e0));
   CK(cudaEventCreate(&e1));
   float best_all = 1e30f;
   int best_mode = mode0;
-  Cfg best_cfg = cfgs[0];
+  bool best_overlap = false;
   for (int mode = mode0; mode < mode1; mode++) {
     c->bt.pairs = mode;
     c->tune_ms[mode] = 1e30f;
-    for (const Cfg& g : cfgs) {
-      c->overlap = g.overlap;
-      c->rebo_grid = g.grid;
+    for (int overlap = 0; overlap <= (lj ? 1 : 0); overlap++) {
+      c->overlap = overlap;
       int rc = evaluate(c);
       if (rc) return rc;
       float best = 1e30f;
@@ -3494,15 +3490,14 @@ static int autotune(mdg_ctx* c)
       if (best < best_all) {
         best_all = best;
         best_mode = mode;
-        best_cfg = g;
+        best_overlap = overlap;
       }
     }
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   c->bt.pairs = best_mode;
-  c->overlap = best_cfg.overlap;
-  c->rebo_grid = best_cfg.grid;
+  c->overlap = best_overlap;
   return read_status(c);
 }
 
@@ -3836,7 +3831,7 @@ int mdg_tuned_launch(mdg_ctx* c, int* overlap, int* rebo_blocks)
 {
   if (!c) return fail(MDG_ERR_ARG, "null context");
   if (overlap) *overlap = c->tuned && c->overlap ? 1 : 0;
-  if (rebo_blocks) *rebo_blocks = (c->prm.potentials & MDG_POT_BRENNER) ? 0 : c->rebo_grid > 0 ? c->rebo_grid : c->rebo_task_blocks;
+  if (rebo_blocks) *rebo_blocks = (c->prm.potentials & MDG_POT_BRENNER) ? 0 : c->rebo_task_blocks;
   return MDG_OK;
 }
 

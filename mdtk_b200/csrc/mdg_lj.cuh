@@ -521,12 +521,12 @@ MDG_HD PairGT<Real> pair_geom(V3 rv, double r, const double4* tan, int lo, int h
   return p;
 }
 
-// Class of one LJ pair seen from atom a: kind 0 (skip: beyond the cutoff or
-// C = 0), 1 (plain: C = 1 and S(t_r) = 0, so E = VLJ) or 2 (special: needs
-// b*_ij or a connectivity gradient); amask = T.mask[a].  The classification
-// is made in double on every path (the adjoint path's pairs are the FP64
-// path's), and the special-pair finder and the plain-pair kernels make it
-// with the same expressions.
+// Class of one far LJ pair (the in-range filter's far list: outside the S(t_r)
+// window) seen from atom a: kind 0 (skip: beyond the cutoff or C = 0), 1 (plain:
+// C = 1, so E = VLJ) or 2 (special: needs a connectivity gradient); amask =
+// T.mask[a].  The classification is made in double on every path (the adjoint
+// path's pairs are the FP64 path's), and the special-pair finder and the
+// plain-pair kernels make it with the same expressions.
 struct LJClass {
   int kind, lo, hi, tb;
   V3 rv;     // x_lo - x_hi
@@ -572,7 +572,7 @@ MDG_HD int lj_kind(double w, bool close)
 
 template <class W>
 MDG_HD LJClass lj_class(const LJParams& P, const CijTableT<W>& T, const State& St, int a, int b, V3 xa, int ta,
-                        unsigned long long amask, bool known_far = false)
+                        unsigned long long amask)
 {
   LJClass c;
   const double4 pb = St.pos[b];
@@ -592,7 +592,7 @@ MDG_HD LJClass lj_class(const LJParams& P, const CijTableT<W>& T, const State& S
   c.C = 1 - w;  // exact for the plain pairs (w = 0); kind 2 takes C from the lower index's table
   if (!(c.C > 0.0)) return c;
   c.r = sqrt(d2);
-  c.kind = lj_kind(w, !known_far && lj_close(P, ta, c.tb, d2));
+  c.kind = lj_kind(w, false);
   return c;
 }
 
@@ -658,16 +658,13 @@ MDG_HD int lj_far_pair_f32(const LJParams& P, const CijTableT<double>& T, const 
   return 1;
 }
 
-// One LJ pair seen from atom a: returns its lj_class kind; for plain pairs
-// adds the own gradient and, at the lower end, the energy.  known_far: the
-// pair is known to lie outside the S(t_r) window (the in-range filter's far
-// list).
+// One far LJ pair seen from atom a: returns its lj_class kind; for plain pairs
+// adds the own gradient and, at the lower end, the energy.
 template <class Real, class S, class W>
 MDG_HD int lj_plain_pair(const LJParams& P, const CijTableT<W>& T, const State& St, int a, int b, V3 xa, int ta,
-                         unsigned long long amask, S& sink, W& e, const double4* tan = nullptr,
-                         bool known_far = false)
+                         unsigned long long amask, S& sink, W& e, const double4* tan)
 {
-  const LJClass c = lj_class(P, T, St, a, b, xa, ta, amask, known_far);
+  const LJClass c = lj_class(P, T, St, a, b, xa, ta, amask);
   if (c.kind != 1) return c.kind;
   // the pair term itself in the arithmetic type
   PairGT<Real> p = pair_geom<Real>(c.rv, c.r, tan, c.lo, c.hi);

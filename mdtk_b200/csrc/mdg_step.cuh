@@ -318,7 +318,6 @@ struct ForceOutT {
   Ws* e_tors;
   Ws* e_lj;
   Ws* dp;           // [n * kNParam] energy derivatives by parameter (adjoint path only)
-  int jt;           // adjoint path: 1 = J^T u, 0 = J u in the gradient's tangents
 };
 typedef ForceOutT<double> ForceOut;
 
