@@ -92,9 +92,8 @@ typedef struct mdg_params {
                          on the first mdg_run (the autotuner) and the fastest kept.  All route the
                          same terms into the same records; results agree to rounding (the kernels
                          may contract multiply-adds differently and mode 3 adds an end's pieces in
-                         two sums).  With the LJ term the launch configuration (stream overlap,
-                         REBO grid) is timed on the first mdg_run in every mode; it never changes
-                         results. */
+                         two sums).  With the LJ term the launch configuration (stream overlap) is
+                         timed on the first mdg_run in every mode; it never changes results. */
 } mdg_params;
 
 /* Fill *p with the defaults: REBO only, FP64, Angstrom/eV/fs, reference cutoffs and skin. */
@@ -281,8 +280,10 @@ int mdg_rebo_compute_noalloc(int n, const double* pos, const int32_t* z, const d
                              int with_torsion, double* energy, double* grad, void* stream);
 
 /* The REBO task mode in use (1 directed, 2 per bond, 3 per bond on lane
- * pairs) and, when the autotuner ran, its timings of one force evaluation in
- * each mode (ms; 0 otherwise).  No reference counterpart. */
+ * pairs) and, when the autotuner ran, its timings in each mode (ms; 0
+ * otherwise): of a whole step of dt 0, or of a force evaluation where the
+ * accelerations were set already (a loaded state, a run after the adjoint).  A
+ * Brenner context reports mode 1.  No reference counterpart. */
 int mdg_task_mode(mdg_ctx* ctx, int* mode, float* ms_directed, float* ms_per_bond, float* ms_split);
 
 /* ---- Thermal bath and adaptive time step ----
@@ -431,9 +432,10 @@ int mdg_snapshots_write(mdg_ctx* ctx, int sys, const char* path, int zip, int te
 int mdg_snapshots_load(mdg_ctx* ctx, int sys, const char* path);
 
 /* The launch configuration the autotuner chose (with the LJ term): overlap = 1
- * when the REBO tasks run on a second stream concurrently with the LJ
- * kernels, rebo_blocks = the REBO task kernel's grid.  No reference
- * counterpart. */
+ * when it chose to run the REBO tasks on a second stream concurrently with the
+ * LJ kernels (0 before it has run, although the force calls of a context that
+ * has not run overlap them too), rebo_blocks = the REBO task kernel's grid, its
+ * resident capacity (0 with Brenner).  No reference counterpart. */
 int mdg_tuned_launch(mdg_ctx* ctx, int* overlap, int* rebo_blocks);
 
 /* Programmatic dependent launch of the step's kernels (default on): each

@@ -432,7 +432,8 @@ class Context:
         _check(lib().mdg_snapshots_load(self.h, sys, os.fsencode(path)))
 
     def tuned_launch(self):
-        """(overlap, rebo_blocks): the autotuner's launch choice."""
+        """(overlap, rebo_blocks): the autotuner's launch choice (overlap 0
+        before it has run) and the REBO task kernel's grid."""
         o = ctypes.c_int()
         b = ctypes.c_int()
         _check(lib().mdg_tuned_launch(self.h, ctypes.byref(o), ctypes.byref(b)))
