@@ -231,6 +231,7 @@ def main():
     ctx.sync()
     mode, ms_dir, ms_pair, ms_split = ctx.task_mode()
     ovl, rblocks = ctx.tuned_launch()
+    # eval_ms_*: the autotuner's time of a whole step of dt 0 in each split
     tuned = {"rebo_task_mode": TASK_MODE_NAMES[mode], "eval_ms_directed": ms_dir, "eval_ms_per_bond": ms_pair,
              "eval_ms_lane_pairs": ms_split, "overlap": bool(ovl), "rebo_blocks": rblocks}
 
@@ -807,10 +808,14 @@ def precision_study(args, local, rank):
 # workload (ethane liquid, 43,688 atoms, step-0 state, seed 1), from the
 # op-counting restatement: `python oracle/opcount.py` (add/mul 1, div/sqrt 4,
 # exp/cos 12, pow 24; energy + gradient = 3 x energy).  rebo_tors = REBO +
-# torsion terms; lj_pairs = the plain LJ pair terms (V_LJ, switches, C_ij
-# path products); lj_special = the b*_ij bond orders of close non-bonded pairs.
-FLOPS_PER_ATOM = {"rebo_tors": 2541.0 + 504.0, "lj_pairs": 5151.5, "lj_special": 5205.5}
-STEP_FLOPS_PER_ATOM = 2541.0 + 504.0 + 10357.0
+# torsion terms; lj_special = the b*_ij bond orders of close non-bonded pairs.
+# lj_pairs is counted from its own form, each far pair once: 14.96 pairs an atom
+# of 31.5 operations (the difference and its square 8, 1/r^2 4, the powers, V and
+# its derivative 12, the gradient 6, the energy and the window's test 1.5), and
+# 47 more for the 6.26 of them inside the cutoff's window (root, two quotients,
+# sine and cosine 36, the products 11).
+FLOPS_PER_ATOM = {"rebo_tors": 2541.0 + 504.0, "lj_pairs": 766.0, "lj_special": 5205.5}
+STEP_FLOPS_PER_ATOM = 2541.0 + 504.0 + 766.0 + 5205.5
 # DRAM read + write bytes per launch of each kernel on this workload, from
 # one ncu capture of the kernel (profiles/, captured with
 #   ncu --set full --clock-control none -k regex:<kernel> -c <few> ...
