@@ -3607,6 +3607,19 @@ static void fill_energy_log(mdg_ctx* c, int nsteps, double* epot, double* etot)
   }
 }
 
+// Room for need doubles in the energy log (without it the log counts as empty:
+// no later call writes through the old size).
+static int elog_reserve(mdg_ctx* c, int64_t need)
+{
+  if (c->elog_cap >= need) return MDG_OK;
+  if (c->d_elog) cudaFree(c->d_elog);
+  c->elog_cap = 0;
+  c->d_elog = dalloc<double>((size_t)need);
+  if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
+  c->elog_cap = need;
+  return MDG_OK;
+}
+
 // nsteps steps after init_first_step; log as step_and_log (rows of 4, or 4 per
 // system, from row 0 of d_elog).  fresh: a new SimLoop::execute (dt_prev = dt);
 // else the continuation of the previous call's loop.
@@ -3616,13 +3629,8 @@ static int step_loop(mdg_ctx* c, int nsteps, double dtf, int log, bool fresh)
   if (rc) return rc;
   if (log) {
     const int64_t need = (int64_t)nsteps * 4 * (log == 2 ? c->nsys : 1);
-    if (c->elog_cap < need) {
-      if (c->d_elog) cudaFree(c->d_elog);
-      c->elog_cap = 0;
-      c->d_elog = dalloc<double>((size_t)need);
-      if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
-      c->elog_cap = need;
-    }
+    rc = elog_reserve(c, need);
+    if (rc) return rc;
     CK(cudaMemsetAsync(c->d_disp_done + 2, 0, sizeof(int), c->stream));
   }
   // Unless profiling, a step and its energy sums are replayed from a CUDA
@@ -3728,12 +3736,8 @@ int mdg_batch_energies(mdg_ctx* c, double* e_sys)
   if (rc) return rc;
   State S = c->S();
   LAUNCH(c, "ekin", k_ekin, nblk(c->n), kThreads, S, c->e_kin);
-  if (c->elog_cap < (int64_t)c->nsys * 4) {
-    if (c->d_elog) cudaFree(c->d_elog);
-    c->d_elog = dalloc<double>((size_t)c->nsys * 4);
-    if (!c->d_elog) return fail(MDG_ERR_CUDA, "cudaMalloc (energy log)");
-    c->elog_cap = (int64_t)c->nsys * 4;
-  }
+  rc = elog_reserve(c, (int64_t)c->nsys * 4);
+  if (rc) return rc;
   rc = sys_energies(c, c->d_elog, nullptr);
   if (rc) return rc;
   std::vector<double> h((size_t)c->nsys * 4);
