@@ -996,6 +996,7 @@ int mdg_set_time_final(mdg_ctx* c, double time_final)
 {
   if (!c) return fail(MDG_ERR_ARG, "null context");
   c->time_final_s = (c->prm.units == MDG_UNITS_CGS) ? time_final : time_final * kFs;
+  c->step_cfg++;  // a captured step of adaptive dt holds it
   return MDG_OK;
 }
 

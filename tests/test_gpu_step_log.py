@@ -59,3 +59,36 @@ def test_rows_of_batch_runs_beside_runs():
         at += k
     for x, y in zip(a.get_state(), b.get_state()):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("energies", [True, False])
+def test_a_final_time_set_between_runs(energies):
+    """Systems of adaptive dt stop at the final time that stands when a run
+    begins, also where an earlier one was in force when the step was captured."""
+    systems = [B.diamond(4, temp_k=t, disp_sigma=0.02, seed=215 + k) for k, t in enumerate((300.0, 1200.0))]
+
+    def load(final):
+        ctx = M.Context(potentials=M.POT_REBO, task_mode=1)
+        ctx.set_batch(systems)
+        ctx.set_adaptive_dt(True, 1.0, 0.5)
+        ctx.set_time_final(final)
+        ctx.set_stop_at_time_final(True)
+        return ctx
+
+    def run(ctx, steps):
+        if energies:
+            ctx.batch_run(steps, 0.5)
+        else:
+            ctx.run(steps, 0.5, energies=False)
+
+    a, b = load(10.0), load(2.0)
+    run(b, 8)  # 2 fs at 0.5 fs a step or less: both systems end on the way
+    assert (b.get_time()[0] >= 2.0).all() and (b.get_time()[0] <= 2.5).all()
+    b.set_time_final(10.0)
+    run(b, 40)
+    run(a, 48)
+    assert (b.get_time()[0] >= 10.0).all() and (b.get_time()[0] <= 10.5).all()
+    assert np.array_equal(a.get_time()[0], b.get_time()[0])
+    # (a stopped system's forces are taken again at its wrapped positions: equal to rounding)
+    for x, y in zip(a.get_state(), b.get_state()):
+        assert np.allclose(x, y, rtol=0, atol=1e-9)
